@@ -68,6 +68,51 @@ int occupancy(const void *fn, int block, size_t smem)
     return nblk;
 }
 
+bool ensure_max_carveout(const void *fn)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, bool> done;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = done.find(std::make_pair(dev, fn));
+    if (it != done.end()) return it->second;
+    const bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         cudaSharedmemCarveoutMaxShared) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    done[std::make_pair(dev, fn)] = ok;
+    return ok;
+}
+
+int tmem_occupancy(const void *fn, int block, size_t smem, int cols, const DeviceInfo &di)
+{
+    static std::mutex mu;
+    static std::map<const void *, std::pair<int, size_t>> regs;  // registers per thread, static shared bytes
+    std::pair<int, size_t> r;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        auto it = regs.find(fn);
+        if (it == regs.end()) {
+            cudaFuncAttributes at{};
+            if (cudaFuncGetAttributes(&at, fn) != cudaSuccess) {
+                cudaGetLastError();
+                return 1;
+            }
+            it = regs.emplace(fn, std::make_pair(at.numRegs, at.sharedSizeBytes)).first;
+        }
+        r = it->second;
+    }
+    // registers come in units of 256 per warp, a quarter of the 64 K with each scheduler
+    const int warps = (block + 31) / 32, warp_regs = round_up(r.first * 32, 256);
+    const int by_regs = 4 * (16384 / warp_regs) / warps;
+    const int by_smem = (int)(di.smem_per_sm / (smem + r.second + di.smem_reserved_cta));
+    int occ = 512 / cols;
+    if (by_regs < occ) occ = by_regs;
+    if (by_smem < occ) occ = by_smem;
+    if (64 / warps < occ) occ = 64 / warps;
+    return occ < 1 ? 1 : (occ > 32 ? 32 : occ);
+}
+
 int launch_tc_forward(int kind, int d, int n, const float *const *mats, int stride, const float *const *in,
                       double *const *out, long long nb, cudaStream_t st, const kronmult_tuning *tune);
 

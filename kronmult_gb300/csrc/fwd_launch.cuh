@@ -3,6 +3,7 @@
 #include <climits>
 #include <cstdint>
 #include <mutex>
+#include "block_kernels.cuh"
 #include "dmma_kernels.cuh"
 #include "fwd_kernels.cuh"
 #include "pair_kernels.cuh"
@@ -254,6 +255,226 @@ bool plan_dmma(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning *
     }
 }
 
+// Whole fibres per thread, a team's consecutive entries summed in registers
+// (fwd_smem_kernel): ts threads per team, at most qmax fibres per thread.
+template <typename T, typename TO>
+bool plan_runs(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning *tune, int ts, int qmax)
+{
+    FwdArgs<T, TO> &a = pl.args;
+    const int n = a.n, d = a.d, N = a.N;
+    const int vpad = round_up(N, 16 / (int)sizeof(T));
+    const int fpad = round_up(d * n * n, 16 / (int)sizeof(T));
+    // two staging slots (asynchronous prefetch of the next entry) unless disabled
+    // or too large for half of the SM's shared memory; FP32 with factors in
+    // shared memory (n >= 6) ping-pongs between vector buffers instead (three
+    // vector buffers, two factor slots)
+    int prefetch = (tune && tune->prefetch == 1) ? 0 : 1;
+    if ((size_t)2 * (vpad + fpad) * sizeof(T) > (size_t)di.max_smem_optin / 2) prefetch = 0;
+    const bool pp_ok = FactorInSmemHost<T>(n) && (size_t)(3 * vpad + 2 * fpad) * sizeof(T) <=
+                                                     (size_t)di.max_smem_optin / 2;
+    // default for FP32 into FP32 outputs (measured 1.5-4.5 % faster on n = 6, 8);
+    // with FP64 outputs the in-place slots measured faster
+    if (pp_ok && ((tune && tune->prefetch == 3) ||
+                  (sizeof(T) == 4 && sizeof(TO) == 4 && (!tune || tune->prefetch == 0))))
+        prefetch = 3;
+    const int team_elems = prefetch == 3 ? 3 * vpad + 2 * fpad : (prefetch ? 2 : 1) * (vpad + fpad);
+    const size_t team_bytes = (size_t)team_elems * sizeof(T);
+    int block = ts >= 256 ? ts : 256;
+    int teams = block / ts;
+    // named barriers 1..15 limit the number of multi-warp teams per CTA
+    while (ts >= 64 && ts < block && teams > 15) {
+        block /= 2;
+        teams = block / ts;
+    }
+    while (teams > 1 && (size_t)teams * team_bytes > (size_t)di.max_smem_optin) {
+        block /= 2;
+        teams = block / ts;
+    }
+    if (block < 32) block = 32, teams = block / ts;
+    const size_t smem = (size_t)teams * team_bytes;
+    if (smem <= (size_t)di.max_smem_optin) {
+        auto fn = fwd_smem_lookup<T, TO>(n, qmax);
+        if (fn && ensure_smem_attr((const void *)fn, smem)) {
+            int per_sm = (tune && tune->ctas_per_sm > 0) ? tune->ctas_per_sm
+                                                         : occupancy((const void *)fn, block, smem);
+            if (per_sm < 1) per_sm = 1;
+            const long long total_teams = (long long)di.sms * per_sm * teams;
+            long long ept = (tune && tune->entries_per_team > 0) ? tune->entries_per_team : 8;
+            if (ept * total_teams > a.nb * 2) ept = (a.nb + total_teams - 1) / total_teams;  // small batches
+            if (ept < 1) ept = 1;
+            if (ept > INT_MAX) ept = INT_MAX;
+            const long long per_cta = ept * teams;
+            const long long grid = (a.nb + per_cta - 1) / per_cta;
+            if (grid <= INT_MAX) {
+                a.team_size = ts;
+                a.teams_per_cta = teams;
+                a.entries_per_team = (int)ept;
+                a.team_elems = team_elems;
+                a.vec_pad = vpad;
+                a.fac_pad = fpad;
+                a.prefetch = prefetch;
+                pl.fn = (const void *)fn;
+                pl.smem_path = true;
+                pl.grid = dim3((unsigned)grid);
+                pl.block = dim3((unsigned)block);
+                pl.smem = smem;
+                return true;
+            }
+        }
+    }
+    return false;
+}
+
+// Team size (threads per entry) of the fibre kernels over F fibres: the smallest team that
+// leaves every thread at most ~2-4 fibres (4 for FP64 n = 6 too: smaller teams keep more
+// entries in flight, measured 5-34 % faster on d = 2..4).
+template <typename T> inline int fibre_team(int n, int F)
+{
+    const int qtarget = (n <= 4 || (n == 6 && sizeof(T) == 8)) ? 4 : 2;
+    int ts = 8;
+    while (ts < 512 && (long long)ts * qtarget < F) ts *= 2;
+    return ts;
+}
+
+// Chunks of the register-block path with FP64 outputs: run sums are kept in FP32 over at
+// most 8 consecutive entries (fewer in small batches; none for n > 8) and added in FP64, so
+// the chunks, and with them the FP32 sums, are fixed by (n, d, batch) alone.  R: teams per
+// SM that the chunk length of a small batch spreads over.
+template <typename TO> bool block_chunks(FwdArgs<float, TO> &a, const DeviceInfo &di, const kronmult_tuning *tune)
+{
+    const int n = a.n, d = a.d;
+    const int forced = tune && tune->entries_per_team > 1 ? tune->entries_per_team : 0;
+    const int ctas = tune && tune->ctas_per_sm > 0 ? tune->ctas_per_sm : 0;
+    long long len = 1;
+    if (n <= 8) {
+        int teams = 0, per_sm = 0;  // per CTA, CTAs per SM
+        if (n == 8 && (d == 3 || d == 4)) {
+            teams = d == 3 ? 8 : 1;
+            per_sm = 3;
+        } else if (n == 4 && d >= 2 && d <= 5) {
+            int ts = 8;
+            while (ts < 256 && ts < a.N / (n * n)) ts *= 2;
+            teams = 256 / ts;
+            per_sm = 3;
+        }
+        if (teams > 0) {
+            const long long R = (long long)di.sms * (ctas ? ctas : per_sm) * teams;
+            len = forced ? forced : 8;
+            if (len * R > a.nb * 2) len = (a.nb + R - 1) / R;
+        } else {
+            FwdPlan<float, TO> p;
+            p.args = a;
+            const int F = a.N / n, ts = fibre_team<float>(n, F), q = (F + ts - 1) / ts;
+            int qmax = 1;
+            while (qmax < q) qmax *= 2;
+            if (qmax > (n <= 4 ? 8 : 4) || !plan_runs<float, TO>(p, di, tune, ts, qmax)) return false;
+            len = p.args.entries_per_team;
+        }
+    }
+    if (len > INT_MAX) return false;
+    a.chunk_len = (int)len;
+    a.chunks = (a.nb + len - 1) / len;
+    return true;
+}
+
+// Gives a kernel that allocates tensor memory the SM's whole shared memory.  The runtime
+// sizes the shared-memory carve-out for the occupancy it computes, and that is one CTA per
+// SM for such kernels: left alone, they run one CTA at a time unless an earlier kernel left
+// a larger carve-out behind (d = 4, n = 4, 5000 entries: 3.8 instead of 14.3 warps per SM).
+bool ensure_max_carveout(const void *fn);
+
+// Resident CTAs per SM of a kernel that holds `cols` tensor-memory columns per CTA: the
+// occupancy call answers 1 for every kernel that allocates tensor memory.
+int tmem_occupancy(const void *fn, int block, size_t smem, int cols, const DeviceInfo &di);
+
+// Where the other FP32 kernels measured faster than the register blocks (us there / in
+// register blocks, at entries).
+template <typename TO> inline bool block_slower(int n, int d, long long nb)
+{
+    if (n == 6 && d == 2) return true;                  // 39.5 / 41.7 at 200000, 8.6 / 11.8 at 30000
+    if (n == 7 && d == 4 && nb < 500) return true;      // few threads per entry: 5.4 / 6.4 at 48
+    if (n == 2 && nb < 20000) return true;              // d = 6: 3.9 / 4.9 at 6000, 10.5 / 8.9 at 30000
+    if (sizeof(TO) == 4) {
+        if (n == 4 && d == 6) return nb < 2500;         // 10.5 / 13.8 at 1000, 40.5 / 38.4 at 6000
+        return n == 8 && d == 4 && nb < 500;            // 4.4 / 5.2 at 48, 31.8 / 22.1 at 2500
+    }
+    // FP64 outputs: chunks of 6-8 entries leave a wave's last teams uneven
+    if (n == 2 || (n == 4 && d == 6)) return true;      // 11.1 / 17.5 (d = 6) and 183 / 193 at 30000
+    if (d == 1 && n <= 6) return true;                  // n = 6: 24.1 / 29.3 at 200000
+    return n == 8 && d == 4 && nb < 4000;               // 33.4 / 37.1 at 2500, 56.3 / 53.6 at 6000
+}
+
+// FP32 register-block plan (fwd_block_kernel) where (n, d) has an instantiation.
+template <typename T, typename TO>
+bool plan_block(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning *tune)
+{
+    if constexpr (sizeof(T) != 4) {
+        return false;
+    } else {
+        FwdArgs<T, TO> &a = pl.args;
+        // a forced team size or one entry per team selects the one-mode-per-step kernels
+        if (tune && (tune->team_size > 0 || tune->entries_per_team == 1 || tune->prefetch == 3)) return false;
+        const BlkPair both = blk_lookup<TO>(a.n, a.d);
+        if (!both.large.fn) return false;
+        if (block_slower<TO>(a.n, a.d, a.nb)) return false;
+        BlkInfo b = both.large;
+        if (both.small.fn) {
+            // one fibre per thread while its groups fill at most one wave of CTAs (n = 8,
+            // d = 3: 3.2 against 5.2 us at 200 entries, 13.1 against 10.8 us at 5000)
+            const BlkInfo &s = both.small;
+            const int occ = tmem_occupancy(s.fn, s.groups * s.group, (size_t)s.groups * s.slot_bytes, s.cols, di);
+            if (a.nb <= (long long)di.sms * occ * s.groups * s.EW) b = s;
+        }
+        if (!ensure_max_carveout(b.fn)) return false;
+        if constexpr (sizeof(TO) == 8) {
+            if (!block_chunks<TO>(a, di, tune)) return false;
+        } else {
+            a.chunks = a.nb;
+            a.chunk_len = 1;
+        }
+        // about 8 warps per SM before groups get more than one team (a group copies and adds for
+        // its teams one after another; more warps cost more than they save at 5000 entries),
+        // and CTAs of fewer groups where that leaves SMs without one
+        const long long spread = (long long)di.sms * 8 * 32 / b.group + 1;
+        long long ew = (a.chunks + spread - 1) / spread;
+        if (ew > b.EW) ew = b.EW;
+        int groups = b.groups;
+        while (groups > 1 && (long long)(groups / 2) * ew * di.sms >= a.chunks) groups /= 2;
+        const int block = groups * b.group;
+        auto smem_of = [&](int slots) { return (size_t)groups * slots * b.slot_bytes; };
+        if (smem_of(1) > (size_t)di.max_smem_optin || !ensure_smem_attr(b.fn, smem_of(1))) return false;
+        int slots = 1, occ = tmem_occupancy(b.fn, block, smem_of(1), b.cols, di);
+        if (a.nb > (long long)di.sms * occ * groups * b.EW || a.chunk_len > 1) {
+            // a second slot (the next entries copied while the current ones are computed)
+            // unless it halves the resident warps
+            if (smem_of(2) <= (size_t)di.max_smem_optin && ensure_smem_attr(b.fn, smem_of(2))) {
+                const int occ2 = tmem_occupancy(b.fn, block, smem_of(2), b.cols, di);
+                if (tune && tune->prefetch > 0 ? tune->prefetch == 2 : 2 * occ2 > occ) slots = 2;
+                if (slots == 2) occ = occ2;
+            }
+        }
+        if (tune && tune->ctas_per_sm > 0 && tune->ctas_per_sm < occ) occ = tune->ctas_per_sm;
+        // at most one wave of CTAs, with equal shares of the chunks
+        long long grid = (a.chunks + groups * ew - 1) / (groups * ew);
+        if (tune && tune->entries_per_team > 1 && sizeof(TO) == 4)
+            grid = (grid + tune->entries_per_team - 1) / tune->entries_per_team;
+        else if (grid > (long long)di.sms * occ)
+            grid = (long long)di.sms * occ;
+        const long long teams = grid * groups * ew;
+        if (grid > INT_MAX || (a.chunks / teams + 1) * a.chunk_len > INT_MAX) return false;
+        a.team_size = (int)ew;
+        a.entries_per_team = (int)(a.chunks / teams);
+        a.teams_per_cta = (int)(groups * ew);
+        a.prefetch = slots == 2;
+        pl.fn = b.fn;
+        pl.smem_path = true;
+        pl.grid = dim3((unsigned)grid);
+        pl.block = dim3((unsigned)block);
+        pl.smem = smem_of(slots);
+        return true;
+    }
+}
+
 // Checks arguments and fills a plan.  Returns cudaSuccess, cudaErrorInvalidValue,
 // or cudaErrorNotSupported (vector too long for any path without a workspace).
 template <typename T, typename TO>
@@ -295,6 +516,9 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
     // ---- FP64 on the tensor path (n = 7, 8, 16 unless tuned otherwise)
     if (plan_dmma<T, TO>(pl, di, tune)) return cudaSuccess;
 
+    // ---- FP32, n and d known at compile time: register blocks
+    if (plan_block<T, TO>(pl, di, tune)) return cudaSuccess;
+
     // ---- register in-place shared-memory path: 2 <= n <= 8, d >= 1
     if (n >= 2 && n <= 8 && d >= 1) {
         const int F = N / n;
@@ -305,11 +529,7 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
             ts = tune->team_size;
             while (ts < 512 && (F + ts - 1) / ts > qcap) ts *= 2;
         } else {
-            // smallest team that leaves every thread at most ~2-4 fibres (4 for FP64
-            // n = 6 too: smaller teams keep more entries in flight, measured 5-34 %
-            // faster on d = 2..4)
-            const int qtarget = (n <= 4 || (n == 6 && sizeof(T) == 8)) ? 4 : 2;
-            while (ts < 512 && (long long)ts * qtarget < F) ts *= 2;
+            ts = fibre_team<T>(n, F);
         }
         // One entry per team (fwd_single_kernel) unless runs are requested: measured
         // fastest for FP64, where the FP64 pipe is the bound and more resident CTAs
@@ -481,9 +701,9 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
                 }
             }
         }
-        // FP32, n = 2 or 4, d >= 2: two modes per shared-memory pass (fwd_pair_kernel)
+        // FP32, n = 2, d >= 2: two modes per shared-memory pass (fwd_pair_kernel)
         if constexpr (sizeof(T) == 4) {
-            const bool want_pair = !single && (n == 2 || n == 4) && d >= 2 && !(tune && tune->prefetch == 1) &&
+            const bool want_pair = !single && n == 2 && d >= 2 && !(tune && tune->prefetch == 1) &&
                                    !(tune && tune->team_size > 0);
             if (want_pair) {
                 const int F2 = N / (n * n);
@@ -523,68 +743,7 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
                 }
             }
         }
-        if (ts_ok && qmax <= qcap) {
-            const int vpad = round_up(N, 16 / (int)sizeof(T));
-            const int fpad = round_up(d * n * n, 16 / (int)sizeof(T));
-            // two staging slots (asynchronous prefetch of the next entry) unless disabled
-            // or too large for half of the SM's shared memory; FP32 with factors in
-            // shared memory (n >= 6) ping-pongs between vector buffers instead (three
-            // vector buffers, two factor slots)
-            int prefetch = (tune && tune->prefetch == 1) ? 0 : 1;
-            if ((size_t)2 * (vpad + fpad) * sizeof(T) > (size_t)di.max_smem_optin / 2) prefetch = 0;
-            const bool pp_ok = FactorInSmemHost<T>(n) && (size_t)(3 * vpad + 2 * fpad) * sizeof(T) <=
-                                                             (size_t)di.max_smem_optin / 2;
-            // default for FP32 into FP32 outputs (measured 1.5-4.5 % faster on n = 6, 8);
-            // with FP64 outputs the in-place slots measured faster
-            if (pp_ok && ((tune && tune->prefetch == 3) ||
-                          (sizeof(T) == 4 && sizeof(TO) == 4 && (!tune || tune->prefetch == 0))))
-                prefetch = 3;
-            const int team_elems = prefetch == 3 ? 3 * vpad + 2 * fpad : (prefetch ? 2 : 1) * (vpad + fpad);
-            const size_t team_bytes = (size_t)team_elems * sizeof(T);
-            int block = ts >= 256 ? ts : 256;
-            int teams = block / ts;
-            // named barriers 1..15 limit the number of multi-warp teams per CTA
-            while (ts >= 64 && ts < block && teams > 15) {
-                block /= 2;
-                teams = block / ts;
-            }
-            while (teams > 1 && (size_t)teams * team_bytes > (size_t)di.max_smem_optin) {
-                block /= 2;
-                teams = block / ts;
-            }
-            if (block < 32) block = 32, teams = block / ts;
-            const size_t smem = (size_t)teams * team_bytes;
-            if (smem <= (size_t)di.max_smem_optin) {
-                auto fn = fwd_smem_lookup<T, TO>(n, qmax);
-                if (fn && ensure_smem_attr((const void *)fn, smem)) {
-                    int per_sm = (tune && tune->ctas_per_sm > 0) ? tune->ctas_per_sm
-                                                                 : occupancy((const void *)fn, block, smem);
-                    if (per_sm < 1) per_sm = 1;
-                    const long long total_teams = (long long)di.sms * per_sm * teams;
-                    long long ept = (tune && tune->entries_per_team > 0) ? tune->entries_per_team : 8;
-                    if (ept * total_teams > nb * 2) ept = (nb + total_teams - 1) / total_teams;  // small batches
-                    if (ept < 1) ept = 1;
-                    if (ept > INT_MAX) ept = INT_MAX;
-                    const long long per_cta = ept * teams;
-                    const long long grid = (nb + per_cta - 1) / per_cta;
-                    if (grid <= INT_MAX) {
-                        a.team_size = ts;
-                        a.teams_per_cta = teams;
-                        a.entries_per_team = (int)ept;
-                        a.team_elems = team_elems;
-                        a.vec_pad = vpad;
-                        a.fac_pad = fpad;
-                        a.prefetch = prefetch;
-                        pl.fn = (const void *)fn;
-                        pl.smem_path = true;
-                        pl.grid = dim3((unsigned)grid);
-                        pl.block = dim3((unsigned)block);
-                        pl.smem = smem;
-                        return cudaSuccess;
-                    }
-                }
-            }
-        }
+        if (ts_ok && qmax <= qcap && plan_runs<T, TO>(pl, di, tune, ts, qmax)) return cudaSuccess;
     }
 
     // ---- large vectors: two passes through the workspace (input left intact)

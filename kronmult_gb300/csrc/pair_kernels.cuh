@@ -909,8 +909,6 @@ template <typename TO> FwdSmemFn<float, TO> fwd_pair_lookup(int nn, int qp);
         switch (nn * 16 + qp) {                                                                        \
         case 2 * 16 + 1: return fwd_pair_kernel<TO, 2, 1>;                                             \
         case 2 * 16 + 2: return fwd_pair_kernel<TO, 2, 2>;                                             \
-        case 4 * 16 + 1: return fwd_pair_kernel<TO, 4, 1>;                                             \
-        case 4 * 16 + 2: return fwd_pair_kernel<TO, 4, 2>;                                             \
         case 8 * 16 + 1: return fwd_pair8_kernel<TO>;                                                  \
         case 4 * 16 + 3: return fwd_tri4_kernel<TO>; /* d = 6: three modes per pass */                 \
         default: return nullptr;                                                                       \

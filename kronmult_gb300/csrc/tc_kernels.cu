@@ -817,7 +817,7 @@ int launch_tc_forward(int kind, int d, int n, const float *const *mats, int stri
     const void *fn = split  ? (const void *)fwd_tc_bf16_kernel<true>
                      : bf16 ? (const void *)fwd_tc_bf16_kernel<false>
                             : (const void *)fwd_tc_kernel<KIND_TF32>;
-    if (!ensure_smem_attr(fn, smem)) return cudaErrorInvalidValue;
+    if (!ensure_smem_attr(fn, smem) || !ensure_max_carveout(fn)) return cudaErrorInvalidValue;
     // runs of 8 consecutive entries per CTA (the fan-in of a typical output group) and as
     // many CTAs as that gives: the hardware keeps as many resident as the shared-memory
     // reservation above allows, and that reservation keeps their TMEM within 512 columns
