@@ -330,6 +330,83 @@ template <typename TO> __device__ __forceinline__ TO blk_out(float v)
     }
 }
 
+// one vector into its slot by SZ threads of rank `rank` < SZ (asynchronous); vectors of
+// B::shifted layouts start blk_shift(src) floats into the slot
+__device__ __forceinline__ int blk_shift(const float *src) { return (int)(reinterpret_cast<uintptr_t>(src) >> 2) & 3; }
+template <typename B, int SZ> __device__ __forceinline__ void blk_copy_vec(float *dst, const float *src, int rank)
+{
+    constexpr int N = B::N;
+    if constexpr (B::shifted) {
+        const int sh = blk_shift(src), end = (N + sh) / 4;
+        const float *s0 = src - sh;
+#pragma unroll
+        for (int i = 0; i < (N / 4 + SZ) / SZ; ++i) {
+            const int c = rank + SZ * i;
+            if ((c > 0 || sh == 0) && c < end) cp_async<16>(dst + 4 * c, s0 + 4 * c);
+        }
+        // the values before the first whole chunk and after the last one
+        if (rank < 3) {
+            if (rank < ((4 - sh) & 3)) cp_async<4>(dst + sh + rank, src + rank);
+            if (rank < ((N + sh) & 3)) cp_async<4>(dst + 4 * end + rank, s0 + 4 * end + rank);
+        }
+    } else if (B::copy16 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+#pragma unroll
+        for (int i = 0; i < (N / 4 + SZ - 1) / SZ; ++i) {
+            const int c = rank + SZ * i;
+            if ((i + 1) * SZ <= N / 4 || c < N / 4) cp_async<16>(dst + B::phys(4 * c), src + 4 * c);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < (N + SZ - 1) / SZ; ++i) {
+            const int p = rank + SZ * i;
+            if ((i + 1) * SZ <= N || p < N) cp_async<4>(dst + B::phys(p), src + p);
+        }
+    }
+}
+
+// Copies the factors of a group's entries: the elements (r, k) of a factor over consecutive
+// lanes, PP factors (of PP teams) at a time.
+template <typename CF> struct BlkFactorLanes {
+    using B = Blk<CF>;
+    static constexpr int P = CF::NN * CF::NN, EW = B::EW, W = B::W;
+    static constexpr int PP = P >= 32 ? 1 : (32 / P < EW ? 32 / P : EW), RR = (P + 31) / 32;
+    int sub, el;
+    size_t off[RR];
+    __device__ __forceinline__ BlkFactorLanes(int lane, int stride)
+    {
+        sub = P >= 32 ? 0 : lane / P;
+        el = P >= 32 ? lane : lane - sub * P;
+#pragma unroll
+        for (int h = 0; h < RR; ++h) off[h] = (el + 32 * h) % CF::NN + (size_t)((el + 32 * h) / CF::NN) * stride;
+    }
+    __device__ __forceinline__ void one(float *dst, const float *m) const
+    {
+#pragma unroll
+        for (int h = 0; h < RR; ++h)
+            if (32 * h + 32 <= P || el + 32 * h < P) cp_async<4>(dst + el + 32 * h, m + off[h]);
+    }
+    // gw: the warp's rank in its group; ptr(i, j): factor i of team j (all lanes call it)
+    template <typename F> __device__ __forceinline__ void copy(float *dst, int gw, int ew, F ptr) const
+    {
+#pragma unroll
+        for (int i = 0; i < CF::D; ++i) {
+            if constexpr (EW <= PP) {  // the warps of a group share the modes
+                if (W == 1 || i % W == gw) {
+                    const float *m = ptr(i, sub < EW ? sub : 0);
+                    if (sub < EW && m) one(dst + sub * B::FS + i * B::P4, m);
+                }
+            } else {
+#pragma unroll 1
+                for (int j0 = gw * PP; j0 < ew; j0 += W * PP) {
+                    const int j = j0 + sub;
+                    const float *m = ptr(i, j < ew ? j : 0);
+                    if (sub < PP && j < ew && m) one(dst + j * B::FS + i * B::P4, m);
+                }
+            }
+        }
+    }
+};
+
 // ---- run sums in tensor memory: each thread's V values in its own lane --------------
 
 template <int NUM> __device__ __forceinline__ void blk_tm_ld1(unsigned a, float *r)
@@ -416,8 +493,8 @@ template <typename TO, typename CF>
 __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_kernel(const FwdArgs<float, TO> a)
 {
     using B = Blk<CF>;
-    constexpr int NN = CF::NN, D = CF::D;
-    constexpr int V = B::V, V0 = B::V0, T = B::T, N = B::N, VS = B::VS, FS = B::FS, P = NN * NN, EW = B::EW, W = B::W;
+    constexpr int D = CF::D;
+    constexpr int V = B::V, V0 = B::V0, T = B::T, N = B::N, VS = B::VS, FS = B::FS, EW = B::EW, W = B::W;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned s_tmem;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -486,42 +563,7 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
         return reinterpret_cast<const float *>(
             __shfl_sync(0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(ptrs[kind / K]), kind % K * EW + j));
     };
-    // one vector by SZ threads of rank `rank` < SZ
-    auto copy_vec = [&](float *dst, const float *src, int rank, auto size) {
-        constexpr int SZ = decltype(size)::value;
-        if constexpr (B::shifted) {
-            const int sh = (int)(reinterpret_cast<uintptr_t>(src) >> 2) & 3, end = (N + sh) / 4;
-            const float *s0 = src - sh;
-#pragma unroll
-            for (int i = 0; i < (N / 4 + SZ) / SZ; ++i) {
-                const int c = rank + SZ * i;
-                if ((c > 0 || sh == 0) && c < end) cp_async<16>(dst + 4 * c, s0 + 4 * c);
-            }
-            // the values before the first whole chunk and after the last one
-            if (rank < 3) {
-                if (rank < ((4 - sh) & 3)) cp_async<4>(dst + sh + rank, src + rank);
-                if (rank < ((N + sh) & 3)) cp_async<4>(dst + 4 * end + rank, s0 + 4 * end + rank);
-            }
-        } else if (B::copy16 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
-#pragma unroll
-            for (int i = 0; i < (N / 4 + SZ - 1) / SZ; ++i) {
-                const int c = rank + SZ * i;
-                if ((i + 1) * SZ <= N / 4 || c < N / 4) cp_async<16>(dst + B::phys(4 * c), src + 4 * c);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < (N + SZ - 1) / SZ; ++i) {
-                const int p = rank + SZ * i;
-                if ((i + 1) * SZ <= N || p < N) cp_async<4>(dst + B::phys(p), src + p);
-            }
-        }
-    };
-    // a factor's elements (r, k) over consecutive lanes, PP factors (of PP teams) at a time
-    constexpr int PP = P >= 32 ? 1 : (32 / P < EW ? 32 / P : EW), RR = (P + 31) / 32;
-    const int fsub = P >= 32 ? 0 : lane / P, fel = P >= 32 ? lane : lane - fsub * P;
-    size_t foff[RR];
-#pragma unroll
-    for (int h = 0; h < RR; ++h) foff[h] = (fel + 32 * h) % NN + (size_t)((fel + 32 * h) / NN) * a.stride;
+    BlkFactorLanes<CF> fl(lane, a.stride);
     // a vector by GS lanes (small teams: several vectors at a time), or by the whole group
     constexpr int pieces = B::shifted || B::copy16 ? (N + 6) / 4 : N;
     constexpr int GS = EW == 1 ? 32 * W : pieces > 16 ? 32 : pieces > 8 ? 16 : pieces > 4 ? 8 : 4;
@@ -530,42 +572,17 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
         float *vdst = base + (size_t)slot * B::SLOT, *fdst = vdst + (EW * VS + 3) / 4 * 4;
         const float *own = ptr_of(0, EW == 1 || !mine ? 0 : team);
         if constexpr (EW == 1) {
-            if (own) copy_vec(vdst, own, grank, std::integral_constant<int, GS>{});
+            if (own) blk_copy_vec<B, GS>(vdst, own, grank);
         } else {
 #pragma unroll 1
             for (int j0 = 0; j0 < ew; j0 += 32 * W / GS) {
                 const int j = j0 + grank / GS;
                 const float *src = ptr_of(0, j < ew ? j : 0);
-                if (j < ew && src) copy_vec(vdst + j * VS, src, lane % GS, std::integral_constant<int, GS>{});
+                if (j < ew && src) blk_copy_vec<B, GS>(vdst + j * VS, src, lane % GS);
             }
         }
-#pragma unroll
-        for (int i = 0; i < D; ++i) {
-            if constexpr (EW <= PP) {  // the warps of a group share the modes
-                if (W == 1 || i % W == gw) {
-                    const float *m = ptr_of(1 + i, fsub < EW ? fsub : 0);
-                    if (fsub < EW && m) {
-#pragma unroll
-                        for (int h = 0; h < RR; ++h)
-                            if (32 * h + 32 <= P || fel + 32 * h < P)
-                                cp_async<4>(fdst + fsub * FS + i * B::P4 + fel + 32 * h, m + foff[h]);
-                    }
-                }
-            } else {
-#pragma unroll 1
-                for (int j0 = gw * PP; j0 < ew; j0 += W * PP) {
-                    const int j = j0 + fsub;
-                    const float *m = ptr_of(1 + i, j < ew ? j : 0);
-                    if (fsub < PP && j < ew && m) {
-#pragma unroll
-                        for (int h = 0; h < RR; ++h)
-                            if (32 * h + 32 <= P || fel + 32 * h < P)
-                                cp_async<4>(fdst + j * FS + i * B::P4 + fel + 32 * h, m + foff[h]);
-                    }
-                }
-            }
-        }
-        return B::shifted ? (int)(reinterpret_cast<uintptr_t>(own) >> 2) & 3 : 0;
+        fl.copy(fdst, gw, ew, [&](int i, int j) { return ptr_of(1 + i, j); });
+        return B::shifted ? blk_shift(own) : 0;
     };
 
     TO *o = count > 0 ? a.out[e0] : nullptr;

@@ -2,6 +2,7 @@
 #include <map>
 #include <mutex>
 #include <utility>
+#include "adj_block.cuh"
 #include "adj_kernels.cuh"
 #include "fwd_launch.cuh"
 
@@ -126,6 +127,40 @@ static int forward_async(int d, int n, const T *const *mats, int stride, const T
     return launch_plan<T, TO>(pl, st);
 }
 
+// FP32 adjoint in register blocks where (n, d) has an instantiation; false: not launched.
+static bool adjoint_block(AdjArgs<float> a, const DeviceInfo &di, cudaStream_t st, int &rc)
+{
+    const AdjBlkInfo b = adj_block_lookup(a.n, a.d);
+    if (!b.fn || !ensure_max_carveout(b.fn)) return false;
+    // teams per group and groups per CTA as in the forward's plan_block
+    const long long spread = (long long)di.sms * 8 * 32 / b.group + 1;
+    long long ew = (a.nb + spread - 1) / spread;
+    if (ew > b.EW) ew = b.EW;
+    int groups = b.groups;
+    while (groups > 1 && (long long)(groups / 2) * ew * di.sms >= a.nb) groups /= 2;
+    const int block = groups * b.group;
+    auto smem_of = [&](int slots) { return (size_t)groups * (slots * b.slot_bytes + b.scratch_bytes); };
+    while (groups > 1 && smem_of(1) > (size_t)di.max_smem_optin) groups /= 2;
+    if (smem_of(1) > (size_t)di.max_smem_optin || !ensure_smem_attr(b.fn, smem_of(1))) return false;
+    int slots = 1, occ = tmem_occupancy(b.fn, block, smem_of(1), b.cols, di);
+    if (a.nb > (long long)di.sms * occ * groups * ew && smem_of(2) <= (size_t)di.max_smem_optin &&
+        ensure_smem_attr(b.fn, smem_of(2))) {
+        const int occ2 = tmem_occupancy(b.fn, block, smem_of(2), b.cols, di);
+        if (occ2 == occ) slots = 2;  // (d = 3, n = 6: 28 us with 3 CTAs of one slot, 32 us with 2 of two)
+    }
+    long long grid = (a.nb + groups * ew - 1) / (groups * ew);
+    if (grid > (long long)di.sms * occ) grid = (long long)di.sms * occ;
+    const long long teams = grid * groups * ew;
+    if (a.nb / teams >= INT_MAX) return false;
+    a.team_size = (int)ew;
+    a.entries_per_team = (int)(a.nb / teams);
+    a.slices = slots;
+    auto fn = reinterpret_cast<void (*)(const AdjArgs<float>)>(const_cast<void *>(b.fn));
+    fn<<<(unsigned)grid, block, smem_of(slots), st>>>(a);
+    rc = (int)cudaGetLastError();
+    return true;
+}
+
 template <typename T>
 static int adjoint_async(int d, int n, const T *const *mats, int stride, const T *const *in, const T *const *gout,
                          T *const *gin, T *const *gmats, int gstride, long long nb, cudaStream_t st,
@@ -143,6 +178,24 @@ static int adjoint_async(int d, int n, const T *const *mats, int stride, const T
     if (cudaGetDevice(&dev) != cudaSuccess) return cudaErrorInvalidDevice;
     const DeviceInfo &di = device_info(dev);
     const int N = (int)Nl, R = N / n, P = n * n;
+    if constexpr (sizeof(T) == 4) {
+        if (!(tune && (tune->team_size > 0 || tune->entries_per_team > 0 || tune->ctas_per_sm > 0))) {
+            AdjArgs<float> b{};
+            b.mats = mats;
+            b.in = in;
+            b.gout = gout;
+            b.gin = gin;
+            b.gmats = gmats;
+            b.nb = nb;
+            b.d = d;
+            b.n = n;
+            b.stride = stride;
+            b.gstride = gstride;
+            b.N = N;
+            int rc = 0;
+            if (adjoint_block(b, di, st, rc)) return rc;
+        }
+    }
     int ts = 0;
     AdjFn<T> fn = nullptr;
     int slices = 1;
