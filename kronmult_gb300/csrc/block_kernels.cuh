@@ -489,7 +489,10 @@ __device__ __forceinline__ void blk_tm_add(unsigned a, float (&y)[NV], bool fres
 }
 
 // a.team_size teams per group are in use (at most EW; one entry at a time per team).
-template <typename TO, typename CF>
+// UNITS: pass 1 of vectors beyond shared memory.  An "entry" is then a unit, one of the
+// split_R chunks of n^D consecutive values of an entry; a.chunks units, their fastest D of
+// a.d axes, and the results are stored to the same place of the entry's workspace.
+template <typename TO, typename CF, bool UNITS = false>
 __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_kernel(const FwdArgs<float, TO> a)
 {
     using B = Blk<CF>;
@@ -506,10 +509,11 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
     // the first `more` teams one more.  FP32 outputs: a chunk is an entry.  FP64 outputs: run
     // sums (in FP32) are cut at chunk edges, chunk_len (at most 8) entries apart.
     constexpr bool kCuts = sizeof(TO) == 8;
+    static_assert(!UNITS || (!kCuts && T >= 8), "units are stored as FP32 by large teams");
     const int ew = a.team_size;
     const long long teams = (long long)gridDim.x * (blockDim.x / (32 * W)) * ew;
     const long long team0 = ((long long)blockIdx.x * (blockDim.x / (32 * W)) + group) * ew;
-    const long long chunks = kCuts ? a.chunks : a.nb;
+    const long long chunks = kCuts || UNITS ? a.chunks : a.nb;
     const int share = a.entries_per_team;
     const long long more = chunks - share * teams;
     auto chunk_of = [&](long long g) { return g * share + (g < more ? g : more); };
@@ -519,11 +523,11 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
     };
     // the most entries of any team, and whether sums outlive an entry
     const int iters = kCuts ? (share + (more > 0 ? 1 : 0)) * a.chunk_len : share + (more > 0 ? 1 : 0);
-    const bool sums = kCuts ? a.chunk_len > 1 : iters > 2;
+    const bool sums = !UNITS && (kCuts ? a.chunk_len > 1 : iters > 2);
     // The next CTA of a kernel that can allocate tensor memory starts on this SM only when
     // this one gives up its right to: at once where nothing is allocated (held to the end,
     // it left one CTA per SM: d = 4, n = 4, 5000 entries 10.0 us).
-    if (!sums && warp == 0) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (!UNITS && !sums && warp == 0) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     if (sums) {
         if (warp == 0) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -554,8 +558,14 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
         for (int r = 0; r < NPR; ++r) {
             const int k = r * K + lkind;
             const bool has = it < lcount && lkind < K && k <= D;
-            const float *const *src = k == 0 ? a.in + (l0 + it) : a.mats + ((l0 + it) * D + (k - 1));
-            ptrs[r] = has ? *src : nullptr;
+            if constexpr (UNITS) {
+                const unsigned u = (unsigned)(l0 + it), e = u / (unsigned)a.split_R;
+                const float *const *src = k == 0 ? a.in + e : a.mats + ((size_t)e * a.d + (a.d - D) + (k - 1));
+                ptrs[r] = has ? *src + (k == 0 ? (size_t)(u - e * a.split_R) * N : 0) : nullptr;
+            } else {
+                const float *const *src = k == 0 ? a.in + (l0 + it) : a.mats + ((l0 + it) * D + (k - 1));
+                ptrs[r] = has ? *src : nullptr;
+            }
         }
     };
     // pointer of kind `kind` (a constant) of team j
@@ -585,7 +595,15 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
         return B::shifted ? blk_shift(own) : 0;
     };
 
-    TO *o = count > 0 ? a.out[e0] : nullptr;
+    auto out_of = [&](long long e) {
+        if constexpr (UNITS) {
+            const unsigned w = (unsigned)e / (unsigned)a.split_R;
+            return a.ws[w] + (size_t)((unsigned)e - w * a.split_R) * N;
+        } else {
+            return a.out[e];
+        }
+    };
+    TO *o = count > 0 ? out_of(e0) : nullptr;
     bool fresh = true;  // the current run starts with this entry
     long long chunk = c0 + 1;  // FP64 outputs: the next chunk and, as an entry of this team, its start
     int cut = kCuts && mine ? (int)(entry_of(chunk) - e0) : 0;
@@ -599,7 +617,7 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
     for (int it = 0; it < iters; ++it) {
         const int slot = slots == 2 ? it & 1 : 0;
         const bool active = it < count;
-        TO *o_next = it + 1 < count ? a.out[e0 + it + 1] : nullptr;
+        TO *o_next = it + 1 < count ? out_of(e0 + it + 1) : nullptr;
         int sh;
         if (slots == 2) {
             cp_async_wait_all();
@@ -630,6 +648,20 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
         float y[V];
 #pragma unroll
         for (int j = 0; j < V0; ++j) blk_split(x[j], y[j], y[V - V0 + j]);
+        if constexpr (UNITS) {
+            if (active) {
+                TO *p = o + t;
+#pragma unroll
+                for (int i = 0; i < L::NG; ++i) {
+                    if (L::has(t, i)) {
+#pragma unroll
+                        for (int m = 0; m < L::NB; ++m) p[T * i + m * L::Q] = y[(i % L::NH) * L::NB + m + (i / L::NH) * V0];
+                    }
+                }
+            }
+            o = o_next;
+            continue;
+        }
         bool last = active && (!sums || o_next != o);
         if constexpr (kCuts) {
             if (active && it + 1 == cut) {
@@ -722,10 +754,10 @@ struct BlkInfo {
     int EW = 0, group = 0, groups = 0, slot_bytes = 0, cols = 0;
 };
 
-template <typename TO, typename CF> BlkInfo blk_info_of()
+template <typename TO, typename CF, bool UNITS = false> BlkInfo blk_info_of()
 {
     using B = Blk<CF>;
-    return BlkInfo{(const void *)fwd_block_kernel<TO, CF>, B::EW, 32 * B::W, B::C, B::SLOT * 4, B::cols};
+    return BlkInfo{(const void *)fwd_block_kernel<TO, CF, UNITS>, B::EW, 32 * B::W, B::C, B::SLOT * 4, B::cols};
 }
 
 // The instantiation for large batches (fn == nullptr where (n, d) has none) and, where

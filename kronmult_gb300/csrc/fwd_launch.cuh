@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <mutex>
 #include "block_kernels.cuh"
+#include "column_kernels.cuh"
 #include "dmma_kernels.cuh"
 #include "fwd_kernels.cuh"
 #include "pair_kernels.cuh"
@@ -119,6 +120,7 @@ template <typename T, typename TO> struct FwdPlan {
     const void *fn2 = nullptr;  // second launch (pass 2 of the two-pass path), same arguments
     dim3 grid2, block2;
     size_t smem2 = 0;
+    bool columns = false;  // both passes in register blocks (launch_columns)
 };
 
 // Fibres per thread the two-pass path's pass-1 kernel is instantiated for, by n.
@@ -197,6 +199,63 @@ bool plan_split(FwdPlan<T, TO> &pl, const DeviceInfo &di)
         return true;
     }
     return false;
+}
+
+// Gives a kernel that allocates tensor memory the SM's whole shared memory.  The runtime
+// sizes the shared-memory carve-out for the occupancy it computes, and that is one CTA per
+// SM for such kernels: left alone, they run one CTA at a time unless an earlier kernel left
+// a larger carve-out behind (d = 4, n = 4, 5000 entries: 3.8 instead of 14.3 warps per SM).
+bool ensure_max_carveout(const void *fn);
+
+// Resident CTAs per SM of a kernel that holds `cols` tensor-memory columns per CTA: the
+// occupancy call answers 1 for every kernel that allocates tensor memory.
+int tmem_occupancy(const void *fn, int block, size_t smem, int cols, const DeviceInfo &di);
+
+// Both passes in register blocks (column_kernels.cuh), for the vectors plan_split takes and
+// pl holds its plan of.  Faster at every shape and batch measured (us, plan_split's kernels /
+// these): n = 8, d = 6 19.9 / 14.0 at 8 entries, 4954 / 2806 at 3905; n = 7, d = 6 2646 / 1507
+// at 3000; n = 8, d = 5 18.0 / 13.9 at 60; n = 2, d = 16 2237 / 725 at 3500.
+template <typename T, typename TO> bool plan_columns(FwdPlan<T, TO> &pl, const DeviceInfo &di)
+{
+    if constexpr (sizeof(T) != 4) {
+        return false;
+    } else {
+        FwdArgs<T, TO> &a = pl.args;
+        const int d1 = a.d - col_axes(a.n);
+        const BlkInfo u = d1 > 0 ? units_lookup(a.n, d1) : BlkInfo{};
+        const ColInfo c = col_lookup<TO>(a.n);
+        if (!u.fn || !c.fn) return false;
+        const long long C = pow_ll(a.n, d1), R = a.N / C, tiles = (C + 31) / 32;
+        const size_t smem1 = (size_t)u.groups * 2 * u.slot_bytes;
+        if (a.nb > INT_MAX / (R > tiles ? R : tiles) || smem1 > (size_t)di.max_smem_optin ||
+            c.smem > di.max_smem_optin || !ensure_smem_attr(u.fn, smem1) || !ensure_smem_attr(c.fn, c.smem) ||
+            !ensure_max_carveout(c.fn))
+            return false;
+        const int block1 = u.groups * u.group, occ1 = occupancy(u.fn, block1, smem1);
+        const int occ2 = tmem_occupancy(c.fn, c.block, c.smem, c.cols, di);
+        if (occ1 < 1) return false;
+        // FP64 outputs: the run sums (in FP32) that plan_split's pass 2 forms
+        a.chunk_len = sizeof(TO) == 8 ? a.entries_per_team : 1;
+        a.chunks = tiles * ((a.nb + a.chunk_len - 1) / a.chunk_len);
+        const long long units = a.nb * R, per = (long long)u.groups * u.EW, warps = c.block / 32;
+        const long long grid1 = (units + per - 1) / per, grid2 = (a.chunks + warps - 1) / warps;
+        a.split_d1 = d1;
+        a.split_C = (int)C;
+        a.split_R = (int)R;
+        a.team_size = u.EW;
+        a.teams_per_cta = (int)per;
+        pl.columns = true;
+        pl.fn = u.fn;
+        pl.grid = dim3((unsigned)(grid1 < (long long)di.sms * occ1 ? grid1 : di.sms * occ1));
+        pl.block = dim3((unsigned)block1);
+        pl.smem = smem1;
+        pl.fn2 = c.fn;
+        pl.grid2 = dim3((unsigned)(grid2 < (long long)di.sms * occ2 ? grid2 : di.sms * occ2));
+        pl.block2 = dim3((unsigned)c.block);
+        pl.smem2 = (size_t)c.smem;
+        a.entries_per_team = (int)(a.chunks / (pl.grid2.x * warps));
+        return true;
+    }
 }
 
 // Whether an FP64 forward of factor size n runs on the FP64 tensor path: forced by
@@ -377,16 +436,6 @@ template <typename TO> bool block_chunks(FwdArgs<float, TO> &a, const DeviceInfo
     return true;
 }
 
-// Gives a kernel that allocates tensor memory the SM's whole shared memory.  The runtime
-// sizes the shared-memory carve-out for the occupancy it computes, and that is one CTA per
-// SM for such kernels: left alone, they run one CTA at a time unless an earlier kernel left
-// a larger carve-out behind (d = 4, n = 4, 5000 entries: 3.8 instead of 14.3 warps per SM).
-bool ensure_max_carveout(const void *fn);
-
-// Resident CTAs per SM of a kernel that holds `cols` tensor-memory columns per CTA: the
-// occupancy call answers 1 for every kernel that allocates tensor memory.
-int tmem_occupancy(const void *fn, int block, size_t smem, int cols, const DeviceInfo &di);
-
 // Where the other FP32 kernels measured faster than the register blocks (us there / in
 // register blocks, at entries).
 template <typename TO> inline bool block_slower(int n, int d, long long nb)
@@ -488,6 +537,7 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
     pl.args = FwdArgs<T, TO>{};
     pl.fn = nullptr;
     pl.fn2 = nullptr;
+    pl.columns = false;
     kronmult_tuning cached{};
     if (!tune) {
         const int code = sizeof(T) == 8 ? KRONMULT_DTYPE_F64
@@ -747,7 +797,10 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
     }
 
     // ---- large vectors: two passes through the workspace (input left intact)
-    if (plan_split<T, TO>(pl, di)) return cudaSuccess;
+    if (plan_split<T, TO>(pl, di)) {
+        plan_columns<T, TO>(pl, di);  // where it can; pl stays as it is otherwise
+        return cudaSuccess;
+    }
 
     // ---- larger still: every mode through input/workspace in global memory, FP64
     // on the tensor path where it is wanted
@@ -806,9 +859,37 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
     return cudaSuccess;
 }
 
+// The two passes of plan_columns.  (Waves of entries whose workspace stays in L2 are slower:
+// n = 8, d = 6, 3905 entries 3340 us with 96 MB at a time, 3571 us with 64 MB, 2770 us at
+// once; every launch ends with a partly empty GPU.)
+template <typename TO> int launch_columns(const FwdPlan<float, TO> &pl, cudaStream_t st)
+{
+    const FwdArgs<float, TO> &a = pl.args;
+    FwdArgs<float, float> u{};
+    u.mats = a.mats;
+    u.in = a.in;
+    u.ws = a.ws;
+    u.d = a.d;
+    u.n = a.n;
+    u.stride = a.stride;
+    u.N = a.N;
+    u.split_R = a.split_R;
+    u.team_size = a.team_size;
+    u.prefetch = 1;
+    u.chunk_len = 1;
+    u.nb = u.chunks = a.nb * a.split_R;
+    u.entries_per_team = (int)(u.chunks / ((long long)pl.grid.x * a.teams_per_cta));
+    reinterpret_cast<void (*)(const FwdArgs<float, float>)>(const_cast<void *>(pl.fn))<<<pl.grid, pl.block, pl.smem, st>>>(u);
+    reinterpret_cast<void (*)(const FwdArgs<float, TO>)>(const_cast<void *>(pl.fn2))<<<pl.grid2, pl.block2, pl.smem2, st>>>(a);
+    return (int)cudaGetLastError();
+}
+
 template <typename T, typename TO> int launch_plan(const FwdPlan<T, TO> &pl, cudaStream_t st)
 {
     if (!pl.fn) return cudaSuccess;
+    if constexpr (sizeof(T) == 4) {
+        if (pl.columns) return launch_columns<TO>(pl, st);
+    }
     if (pl.smem_path) {
         auto fn = reinterpret_cast<void (*)(const FwdArgs<T, TO>)>(const_cast<void *>(pl.fn));
         fn<<<pl.grid, pl.block, pl.smem, st>>>(pl.args);

@@ -1,6 +1,8 @@
 // Forward kernels for FP32 vectors beyond shared memory: two passes through the
 // workspace (the declarations of their lookups live in fwd_kernels.cuh; the
-// instantiation units that serve FP32 storage include this file).
+// instantiation units that serve FP32 storage include this file).  Run for the (n, d)
+// that column_kernels.cuh has no instantiation for: n = 2, d > 18; n = 3, d > 11; n = 4,
+// d > 9; n = 5..8 with d1 too large for it, and batches beyond its 32-bit unit counts.
 #pragma once
 #include "fwd_kernels.cuh"
 
