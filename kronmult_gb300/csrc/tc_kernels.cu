@@ -28,9 +28,17 @@
 // [A_i 0; 0 A_i], so the operand carries no zero padding.  TF32 (fwd_tc_kernel; K = 8
 // per MMA) keeps the backward order and the K-major operand, written element by element.
 //
-// One CTA = one warpgroup (128 threads) works on one entry at a time; several
-// CTAs per SM overlap the input loads.  Consecutive entries with the same
-// output pointer are summed in tensor memory and added with FP64 atomics.
+// One CTA of up to four warps works on one entry at a time; several CTAs per SM overlap the
+// input loads.  Consecutive entries with the same output pointer are summed in tensor memory
+// and added with FP64 atomics.
+//
+// What bounds it: the chain of steps of an entry (copy, convert, then per mode MMA, wait,
+// TMEM load, store, barrier) times the CTAs that shared memory admits (d = 4: 6 for TF32, 8
+// for BF16).  Hence d at compile time, operands that stay in uniform registers for the MMAs,
+// one barrier per mode, all TMEM loads of a mode before one wait, and exact integer
+// conversion of the sums to FP64.  FP32 storage, FP64 outputs, 32768 entries of d = 4: TF32
+// 224 -> 170 us (3.9 TB/s; shared-memory pipe 63 % busy), BF16 140 -> 128 us, split BF16 225
+// -> 201 us; 200000 entries of d = 2: TF32 349 -> 110, BF16 302 -> 111, split 466 -> 181 us.
 //
 // Every wait on an mbarrier is bounded; on timeout the kernel records an error
 // code in a device word (kronmult_device_error) and leaves after freeing its
@@ -45,7 +53,6 @@ __device__ unsigned int g_tc_error = 0;  // 0 = ok; otherwise the code of the fi
 
 namespace {
 
-constexpr int kTcThreads = 128;
 constexpr int kTileRows = 128;               // fibres per MMA (M)
 constexpr int kTileBytes = kTileRows * 32;   // one K-major tile: 128 rows x 32 bytes
 constexpr int kBBytes = 16 * 32;             // one factor operand: 16 rows x 32 bytes
@@ -87,7 +94,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo = 128
 // later.  The two 16-byte halves of a row then sit 64 bytes apart modulo the 128-byte
 // bank row, so the epilogue's stores (consecutive lanes = consecutive rows, both
 // halves) and the staging conversion hit distinct banks.
-__device__ __forceinline__ uint32_t a_lbo(int tiles) { return (uint32_t)tiles * 2048u + 64u; }
 __device__ __forceinline__ uint32_t a_offset(uint32_t row, uint32_t kbyte, uint32_t lbo)
 {
     return (row >> 3) * 128u + (kbyte >> 4) * lbo + (row & 7u) * 16u + (kbyte & 15u);
@@ -101,29 +107,31 @@ template <int KIND, bool A_MN_MAJOR = false> __device__ __forceinline__ constexp
            ((A_MN_MAJOR ? 1u : 0u) << 15) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
 }
 
+// The lane that issues MMAs and their commits.  Whole warps run the issuing code with warp-
+// uniform operands, predicated on that lane (in a branch of one thread the operands went
+// through vector registers: 600 cycles per mode, now 100).
+__device__ __forceinline__ uint32_t elect_lane()
+{
+    uint32_t leader;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(leader));
+    return leader;
+}
+
+// D (+)= A B where `leader`; BF16: A MN-major (the vector), B K-major (the factor)
 template <int KIND>
-__device__ __forceinline__ void mma(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
+__device__ __forceinline__ void mma(uint32_t leader, uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
 {
     if constexpr (KIND == KIND_TF32) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dtmem),
-            "l"(adesc), "l"(bdesc), "r"(instr_desc<KIND>()), "r"(accumulate));
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dtmem),
+            "l"(adesc), "l"(bdesc), "r"(instr_desc<KIND>()), "r"(accumulate), "r"(leader));
     } else {
         asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dtmem),
-            "l"(adesc), "l"(bdesc), "r"(instr_desc<KIND>()), "r"(accumulate));
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dtmem),
+            "l"(adesc), "l"(bdesc), "r"(instr_desc<KIND_BF16, true>()), "r"(accumulate), "r"(leader));
     }
-}
-
-// BF16 MMA with an MN-major A operand (the vector) and a K-major B operand (the factor)
-__device__ __forceinline__ void mma_bf16_mn(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dtmem),
-        "l"(adesc), "l"(bdesc), "r"(instr_desc<KIND_BF16, true>()), "r"(accumulate));
 }
 
 // 8 FP32 values rounded to BF16 (nearest even), packed in order into 16 bytes
@@ -181,10 +189,12 @@ __device__ __forceinline__ void octet_transpose(float (&v)[8], int lane)
     }
 }
 
-__device__ __forceinline__ void mma_commit(uint32_t mbar)
+__device__ __forceinline__ void mma_commit(uint32_t leader, uint32_t mbar)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
-                 : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(mbar), "r"(leader)
+        : "memory");
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase, unsigned limit = kWaitLimit)
@@ -205,20 +215,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase, unsigne
 // 16 consecutive columns of this warp's 32 lanes: the two tiles of one block
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v0)[8], float (&v1)[8])
 {
-    uint32_t r[16];
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "=f"(v0[0]), "=f"(v0[1]), "=f"(v0[2]), "=f"(v0[3]), "=f"(v0[4]), "=f"(v0[5]), "=f"(v0[6]), "=f"(v0[7]),
+          "=f"(v1[0]), "=f"(v1[1]), "=f"(v1[2]), "=f"(v1[3]), "=f"(v1[4]), "=f"(v1[5]), "=f"(v1[6]), "=f"(v1[7])
         : "r"(taddr));
+}
+// no use of loaded values before the wait
+template <int NT> __device__ __forceinline__ void tmem_wait_ld(float (&v)[NT][8])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        v0[j] = __uint_as_float(r[j]);
-        v1[j] = __uint_as_float(r[8 + j]);
-    }
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) asm volatile("" : "+f"(v[t][j]));
 }
 
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -272,23 +284,49 @@ struct TcArgs {
     const float *const *in;
     double *const *out;
     long long nb;
-    int d, stride, N, tiles, tmem_cols, entries_per_cta;
+    int stride, entries_per_chunk;
+};
+
+// d modes: sizes known at compile time.  A CTA has no more warps than the vector has fibres
+// in tensor-memory lanes (the others' instructions are wasted: d = 2, 200000 entries, TF32,
+// 198 us with four warps, 110 with one; d = 3, 60000 entries, 89 with four, 65 with two).  Two
+// warpgroups for d = 4 were slower (TF32, 32768 entries: 220 against 170 us).
+template <int D> struct TcShape {
+    static constexpr int d = D, N = 1 << (3 * D), F = N / 8;
+    static constexpr int threads = F >= 128 ? 128 : F > 32 ? F : 32;
+    static constexpr int copier = threads > 32 ? 32 : 0;  // issues bulk copies (warp 0 issues MMAs)
+    static constexpr int tiles = (F + kTileRows - 1) / kTileRows, pairs = (tiles + 1) / 2;
+    static constexpr int cols = 32 * pairs;  // tensor-memory columns: mode output + run sums
+    static constexpr int fac_slots = (D * 64 + threads - 1) / threads;  // factor elements per thread
+};
+
+// A CTA's entries: chunks of entries_per_chunk consecutive ones, gridDim.x chunks apart.
+// Run sums end with their chunk.  (One chunk per CTA: a CTA of a kernel that allocates tensor
+// memory starts on an SM only when the one before has given up its right to, which left the
+// small vectors waiting for CTA starts.)
+struct TcWalk {
+    long long e;  // the current entry (a.nb or beyond: none)
+    int left;     // entries left in its chunk, itself included
+    __device__ __forceinline__ TcWalk next(const TcArgs &a) const
+    {
+        if (left > 1) return TcWalk{e + 1, left - 1};
+        return TcWalk{e + 1 + (long long)(gridDim.x - 1) * a.entries_per_chunk, a.entries_per_chunk};
+    }
 };
 
 // per-thread pointers of one entry, loaded one entry ahead of the copies that use them
-constexpr int kTcFacSlots = 2;  // factor elements per thread: d*64 <= 256 = 2 x 128 threads
-struct TcPtrs {
+template <int D> struct TcPtrs {
     const float *src;
-    const float *mat[kTcFacSlots];
+    const float *mat[TcShape<D>::fac_slots];
 };
 
-__device__ __forceinline__ void tc_load_ptrs(TcPtrs &p, const TcArgs &a, long long e, int tid)
+template <int D> __device__ __forceinline__ void tc_load_ptrs(TcPtrs<D> &p, const TcArgs &a, long long e, int tid)
 {
     p.src = a.in[e];
 #pragma unroll
-    for (int s = 0; s < kTcFacSlots; ++s) {
-        const int idx = tid + s * kTcThreads;
-        p.mat[s] = idx < a.d * 64 ? a.mats[e * a.d + (idx >> 6)] : nullptr;
+    for (int s = 0; s < TcShape<D>::fac_slots; ++s) {
+        const int idx = tid + s * TcShape<D>::threads;
+        p.mat[s] = idx < D * 64 ? a.mats[e * D + (idx >> 6)] : nullptr;
     }
 }
 
@@ -300,13 +338,16 @@ __device__ __forceinline__ void tc_load_ptrs(TcPtrs &p, const TcArgs &a, long lo
 // elements with cp.async and thread 0 completes the barrier's phase without bytes.
 // Either way the staging barrier completes exactly one phase per entry.  The factor
 // loads are plain loads consumed one entry later, so their latency is hidden too.
-__device__ __forceinline__ void tc_stage_async(float *raw, float (&fv)[kTcFacSlots], const TcPtrs &p,
+// Returns whether it was the bulk copy.
+template <int D>
+__device__ __forceinline__ bool tc_stage_async(float *raw, float (&fv)[TcShape<D>::fac_slots], const TcPtrs<D> &p,
                                                const TcArgs &a, int tid, uint32_t sbar)
 {
-    const int N = a.N;
-    const unsigned bytes = (unsigned)N * 4u;
-    if (((reinterpret_cast<uintptr_t>(p.src) & 15u) == 0) && ((bytes & 15u) == 0)) {
-        if (tid == 0) {
+    constexpr int N = TcShape<D>::N;
+    constexpr unsigned bytes = (unsigned)N * 4u;
+    const bool bulk = (reinterpret_cast<uintptr_t>(p.src) & 15u) == 0;
+    if (bulk) {
+        if (tid == TcShape<D>::copier) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sbar), "r"(bytes)
                          : "memory");
             asm volatile(
@@ -316,111 +357,115 @@ __device__ __forceinline__ void tc_stage_async(float *raw, float (&fv)[kTcFacSlo
                 : "memory");
         }
     } else {
-        for (int q = tid; q < N; q += kTcThreads) cp_async<4>(raw + q, p.src + q);
-        if (tid == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sbar) : "memory");
+        for (int q = tid; q < N; q += TcShape<D>::threads) cp_async<4>(raw + q, p.src + q);
+        if (tid == TcShape<D>::copier) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sbar) : "memory");
     }
     cp_async_commit();
 #pragma unroll
-    for (int s = 0; s < kTcFacSlots; ++s) {
-        const int idx = tid + s * kTcThreads;
-        if (idx < a.d * 64) {
+    for (int s = 0; s < TcShape<D>::fac_slots; ++s) {
+        const int idx = tid + s * TcShape<D>::threads;
+        if (idx < D * 64) {
             const int r = idx & 7, k = (idx >> 3) & 7;
             fv[s] = __ldg(p.mat[s] + r + (size_t)k * a.stride);
         }
     }
+    return bulk;
 }
 
-template <int KIND> __global__ void __launch_bounds__(kTcThreads, 6) fwd_tc_kernel(const TcArgs a)
+template <int D> __global__ void __launch_bounds__(TcShape<D>::threads, D == 4 ? 6 : 16) fwd_tc_kernel(const TcArgs a)
 {
+    constexpr int KIND = KIND_TF32;
+    using S = TcShape<D>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int N = a.N, F = N / 8, d = a.d;
+    constexpr int N = S::N, F = S::F, d = D, tiles = S::tiles, blocks = S::pairs;  // 16-column accumulator blocks, two tiles each
     // shared memory: one raw staging slot for the vector, operand A, operands B, barriers.
     // The slot is refilled with the next entry as soon as this entry's operands are built.
     float *raw = reinterpret_cast<float *>(smem_raw);
     unsigned char *xs = reinterpret_cast<unsigned char *>(raw + N);  // tiles x 4 KB
-    unsigned char *bs = xs + (size_t)a.tiles * kTileBytes + 64;            // d x 512 B: [A_i^T | 0]
+    unsigned char *bs = xs + (size_t)tiles * kTileBytes + 64;            // d x 512 B: [A_i^T | 0]
     unsigned char *bs2 = bs + (size_t)d * kBBytes;                         // d x 512 B: [0 | A_i^T]
     uint64_t *mbar = reinterpret_cast<uint64_t *>(bs2 + (size_t)d * kBBytes);  // MMA completion
     uint64_t *sbar = mbar + 1;                                                  // staging completion
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + 2);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
-    long long e = (long long)blockIdx.x * a.entries_per_cta;
-    const long long e_end = min(e + (long long)a.entries_per_cta, a.nb);
-    if (e >= e_end) return;
+    const long long nb = a.nb;
+    TcWalk w{(long long)blockIdx.x * a.entries_per_chunk, a.entries_per_chunk};  // the entry being computed
+    if (w.e >= nb) return;
+    TcWalk w1 = w.next(a);  // the entry staged after it
 
     // operands zeroed once: the zero half of each B (rows 8..15 of [A^T | 0], rows 0..7 of
     // [0 | A^T]) and, for BF16, the K 8..15 half of A stay zero
-    for (int v = tid; v < (a.tiles * kTileBytes + 64 + 2 * d * kBBytes) / 16; v += kTcThreads)
+    for (int v = tid; v < (tiles * kTileBytes + 64 + 2 * d * kBBytes) / 16; v += S::threads)
         reinterpret_cast<int4 *>(xs)[v] = make_int4(0, 0, 0, 0);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(a.tmem_cols)
+                     "n"(S::cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     const uint32_t sbar_a = smem_u32(sbar);
-    if (tid == 0) {
+    if (tid == S::copier) {  // the thread that uses the staging barrier before the others see it
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar_a) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    TcPtrs nxt;
-    float fv[kTcFacSlots] = {0.f, 0.f};  // factor elements of the entry staged last
-    tc_load_ptrs(nxt, a, e, tid);
-    tc_stage_async(raw, fv, nxt, a, tid, sbar_a);
-    if (e + 1 < e_end) tc_load_ptrs(nxt, a, e + 1, tid);
+    TcPtrs<D> nxt;
+    float fv[S::fac_slots] = {};  // factor elements of the entry staged last
+    tc_load_ptrs<D>(nxt, a, w.e, tid);
+    const bool bulk0 = tc_stage_async<D>(raw, fv, nxt, a, tid, sbar_a);
+    if (w1.e < nb) tc_load_ptrs<D>(nxt, a, w1.e, tid);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const int blocks = (a.tiles + 1) / 2;        // 16-column accumulator blocks, two tiles each
     const uint32_t tacc = tmem + 16u * blocks;   // run accumulator after the mode output
     const uint32_t mbar_a = smem_u32(mbar);
     const uint32_t xs_a = smem_u32(xs), bs_a = smem_u32(bs), bs2_a = smem_u32(bs2);
-    const uint32_t lboa = a_lbo(a.tiles);  // A operand: k-chunk-1 core matrices this far after chunk 0
+    constexpr uint32_t lboa = (uint32_t)tiles * 2048u + 64u;  // A operand: k-chunk-1 core matrices this far after chunk 0
+    const uint32_t leader = elect_lane();  // of each warp; warp 0's issues the MMAs
     uint32_t phase = 0, sphase = 0;
     bool failed = false;
     bool staging = true;  // a staging copy is in flight whose phase has not been waited for
     double *cur = nullptr;
-    constexpr int MAXT = 4;  // tiles per entry (N <= 4096)
 
     // run sum (TMEM accumulator) -> FP64 atomics into `dst`
     auto flush = [&](double *dst) {
         auto add_tile = [&](int t, const float (&v)[8]) {
             const int c = t * kTileRows + warp * 32 + lane;
-            if (t < a.tiles && c < F)
+            if (c < F)
 #pragma unroll
-                for (int r = 0; r < 8; ++r) red_add_f64(dst + c + r * F, (double)v[r]);
+                for (int r = 0; r < 8; ++r) red_add_f64(dst + c + r * F, blk_out<double>(v[r]));
         };
 #pragma unroll
-        for (int j = 0; j < MAXT / 2; ++j) {
-            if (j < blocks) {
-                float v0[8], v1[8];
-                tmem_ld16(tacc + ((uint32_t)(warp * 32) << 16) + 16u * j, v0, v1);
-                tmem_wait_ld();
-                add_tile(2 * j, v0);
-                add_tile(2 * j + 1, v1);
-            }
+        for (int j = 0; j < blocks; ++j) {
+            float v[2][8];
+            tmem_ld16(tacc + ((uint32_t)(warp * 32) << 16) + 16u * j, v[0], v[1]);
+            tmem_wait_ld(v);
+            add_tile(2 * j, v[0]);
+            add_tile(2 * j + 1, v[1]);
         }
     };
 
-    for (; e < e_end; ++e) {
-        double *o = a.out[e];
+    bool ok = true;      // this warp's waits so far; the CTA agrees on it at the next barrier
+    bool bulk = bulk0;   // how the entry being computed was staged
+    for (; w.e < nb; w = w1, w1 = w.next(a)) {
+        double *o = a.out[w.e];
         cp_async_wait_all();
-        const bool staged = mbar_wait(sbar_a, sphase);  // the slot's bulk copy (or its empty phase)
-        if (__syncthreads_or(!staged)) {  // slot complete for every thread; previous MMAs done
-            if (tid == 0) atomicCAS(&g_tc_error, 0u, 1u);
-            failed = true;
-            break;
+        ok = ok && mbar_wait(sbar_a, sphase);  // the slot's bulk copy (or its empty phase)
+        ok = __all_sync(0xffffffffu, ok);
+        // a bulk copy is complete for whoever waited for it, copies by threads need a barrier;
+        // the MMAs that read the operands are done for every thread (each waited for them)
+        if (!bulk) __syncthreads();
+        if (ok) {
+            sphase ^= 1u;
+            staging = false;
         }
-        sphase ^= 1u;
-        staging = false;
         // operands: B_i[row r][k] = A_i(r, k) (and row r + 8 of the second copy); input
         // natural index p = k + 8c -> A row c, column k
 #pragma unroll
-        for (int s = 0; s < kTcFacSlots; ++s) {
-            const int v = tid + s * kTcThreads;
+        for (int s = 0; s < S::fac_slots; ++s) {
+            const int v = tid + s * S::threads;
             if (v < d * 64) {
                 const int i = v >> 6, r = v & 7, k = (v >> 3) & 7;
                 put<KIND>(bs + (size_t)i * kBBytes, r, k, fv[s]);
@@ -429,7 +474,8 @@ template <int KIND> __global__ void __launch_bounds__(kTcThreads, 6) fwd_tc_kern
         }
         // natural position p = k + 8c -> operand row c, column k: the 4 values of a float4
         // are one 16-byte half of a core-matrix row
-        for (int q = tid; q < N / 4; q += kTcThreads) {
+#pragma unroll
+        for (int q = tid; q < N / 4; q += S::threads) {
             const float4 v4 = *reinterpret_cast<const float4 *>(raw + 4 * q);
             const uint32_t c = q >> 1, kbyte = (q & 1) * 16;
             *reinterpret_cast<float4 *>(xs + a_offset(c, kbyte, lboa)) =
@@ -437,37 +483,38 @@ template <int KIND> __global__ void __launch_bounds__(kTcThreads, 6) fwd_tc_kern
         }
         // the run continues when this entry adds into the same output as the previous one;
         // otherwise the previous run's sum leaves TMEM before the last mode overwrites it
-        const bool cont = (o == cur);
-        if (!cont && cur != nullptr) flush(cur);
+        const bool cont = o == cur && w.left < a.entries_per_chunk;
+        if (!cont && cur != nullptr && ok) flush(cur);
         cur = o;
         fence_async_smem();  // the staging slot has been read (generic proxy) before the bulk copy refills it
         tc_fence_before();
-        __syncthreads();
-        if (e + 1 < e_end) {
-            tc_stage_async(raw, fv, nxt, a, tid, sbar_a);
+        if (__syncthreads_or(!ok)) {
+            failed = true;
+            break;
+        }
+        if (w1.e < nb) {
+            bulk = tc_stage_async<D>(raw, fv, nxt, a, tid, sbar_a);
             staging = true;
-            if (e + 2 < e_end) tc_load_ptrs(nxt, a, e + 2, tid);
+            const TcWalk w2 = w1.next(a);
+            if (w2.e < nb) tc_load_ptrs<D>(nxt, a, w2.e, tid);
         }
 
         for (int i = d - 1; i >= 0; --i) {
-            if (tid == 0) {
+            if (warp == 0) {
                 tc_fence_after();
                 const uint32_t dst = i > 0 ? tmem : tacc;
                 const uint32_t accumulate = (i == 0 && cont) ? 1u : 0u;
                 // even tile: columns 0..7 of its block (overwriting, or adding to the run);
                 // odd tile: columns 8..15, always added (the even tile's B zeroed them)
-                for (int t = 0; t < a.tiles; ++t)
-                    mma<KIND>(dst + 16u * (uint32_t)(t >> 1), smem_desc(xs_a + t * 2048u, lboa, 128u),
+#pragma unroll
+                for (int t = 0; t < tiles; ++t)
+                    mma<KIND>(leader, dst + 16u * (uint32_t)(t >> 1), smem_desc(xs_a + t * 2048u, lboa, 128u),
                               smem_desc(((t & 1) ? bs2_a : bs_a) + i * kBBytes), (t & 1) ? 1u : accumulate);
-                mma_commit(mbar_a);
+                mma_commit(leader, mbar_a);
             }
-            const bool ok = mbar_wait(mbar_a, phase);
-            // the decision to leave must be uniform: the TMEM loads below are warp-collective
-            if (__syncthreads_or(!ok)) {
-                if (tid == 0) atomicCAS(&g_tc_error, 0u, 1u);
-                failed = true;
-                break;
-            }
+            // uniform over the warp (the TMEM loads below are warp-collective), over the CTA at
+            // the next barrier
+            ok = __all_sync(0xffffffffu, mbar_wait(mbar_a, phase));
             phase ^= 1u;
             tc_fence_after();
             if (i > 0) {
@@ -476,7 +523,7 @@ template <int KIND> __global__ void __launch_bounds__(kTcThreads, 6) fwd_tc_kern
                 // tiles) at a time keeps 16 values per thread live
                 auto store_tile = [&](int t, const float (&v)[8]) {
                     const int c = t * kTileRows + warp * 32 + lane;
-                    if (t < a.tiles && c < F) {
+                    if (c < F) {
                         if (F >= 64) {
                             // F/8 a multiple of 8: row p/8 = c/8 + r*F/8 keeps its position in
                             // the 8-row group and moves r*F/64 groups, 2F bytes per r
@@ -493,22 +540,26 @@ template <int KIND> __global__ void __launch_bounds__(kTcThreads, 6) fwd_tc_kern
                         }
                     }
                 };
+                float v[2 * blocks][8];
 #pragma unroll
-                for (int j = 0; j < MAXT / 2; ++j) {
-                    if (j < blocks) {
-                        float v0[8], v1[8];
-                        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + 16u * j, v0, v1);
-                        tmem_wait_ld();
-                        store_tile(2 * j, v0);
-                        store_tile(2 * j + 1, v1);
-                    }
-                }
+                for (int j = 0; j < blocks; ++j)
+                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + 16u * j, v[2 * j], v[2 * j + 1]);
+                tmem_wait_ld(v);
+#pragma unroll
+                for (int t = 0; t < 2 * blocks; ++t) store_tile(t, v[t]);
                 fence_async_smem();
                 tc_fence_before();
-                __syncthreads();
+                if (__syncthreads_or(!ok)) {
+                    failed = true;
+                    break;
+                }
             }
         }
         if (failed) break;
+    }
+    if (!ok || failed) {
+        failed = true;
+        if (lane == 0) atomicCAS(&g_tc_error, 0u, 1u);
     }
     cp_async_wait_all();
     // leaving early with a bulk copy still in flight: one more bounded wait for it, so
@@ -519,7 +570,7 @@ template <int KIND> __global__ void __launch_bounds__(kTcThreads, 6) fwd_tc_kern
     __syncthreads();
     tc_fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(S::cols) : "memory");
 }
 
 // BF16 forward (layout and mode order in the file comment).  Same pipeline as
@@ -531,12 +582,12 @@ template <int KIND> __global__ void __launch_bounds__(kTcThreads, 6) fwd_tc_kern
 // accumulator, x_hi.A_hi + x_lo.A_hi + x_hi.A_lo (the lo.lo term, 2^-16 relative, is
 // dropped): about 16 significand bits per product instead of 8.  The hi and lo vector
 // operands and factor operands sit side by side in the same layouts.
-template <bool SPLIT>
-__global__ void __launch_bounds__(kTcThreads, SPLIT ? 5 : 8) fwd_tc_bf16_kernel(const TcArgs a)
+template <bool SPLIT, int D>
+__global__ void __launch_bounds__(TcShape<D>::threads, D < 4 ? 16 : SPLIT ? 5 : 8) fwd_tc_bf16_kernel(const TcArgs a)
 {
+    using S = TcShape<D>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int N = a.N, F = N / 8, d = a.d;
-    const int pairs = (a.tiles + 1) / 2;
+    constexpr int N = S::N, F = S::F, d = D, tiles = S::tiles, pairs = S::pairs;
     constexpr int kParts = SPLIT ? 2 : 1;
     float *raw = reinterpret_cast<float *>(smem_raw);                          // staging slot, N floats
     unsigned char *xs = reinterpret_cast<unsigned char *>(raw + N);           // pairs x kPairBytes (hi)
@@ -546,33 +597,34 @@ __global__ void __launch_bounds__(kTcThreads, SPLIT ? 5 : 8) fwd_tc_bf16_kernel(
     uint64_t *mbar = reinterpret_cast<uint64_t *>(bs + (size_t)kParts * d * kBf16B);  // MMA completion
     uint64_t *sbar = mbar + 1;                                                // staging completion
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + 2);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
 
-    long long e = (long long)blockIdx.x * a.entries_per_cta;
-    const long long e_end = min(e + (long long)a.entries_per_cta, a.nb);
-    if (e >= e_end) return;
+    const long long nb = a.nb;
+    TcWalk w{(long long)blockIdx.x * a.entries_per_chunk, a.entries_per_chunk};  // the entry being computed
+    if (w.e >= nb) return;
+    TcWalk w1 = w.next(a);  // the entry staged after it
 
     // operands zeroed once: fibres beyond F, the odd K half of an unpaired tile and the
     // off-diagonal blocks of the factor operands stay zero
-    for (int v = tid; v < (int)(kParts * pairs * kPairBytes + 64 + kParts * d * kBf16B) / 16; v += kTcThreads)
+    for (int v = tid; v < (int)(kParts * pairs * kPairBytes + 64 + kParts * d * kBf16B) / 16; v += S::threads)
         reinterpret_cast<int4 *>(xs)[v] = make_int4(0, 0, 0, 0);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(a.tmem_cols)
+                     "n"(S::cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     const uint32_t sbar_a = smem_u32(sbar);
-    if (tid == 0) {
+    if (tid == S::copier) {  // the thread that uses the staging barrier before the others see it
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar_a) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    TcPtrs nxt;
-    float fv[kTcFacSlots] = {0.f, 0.f};  // factor elements of the entry staged last
-    tc_load_ptrs(nxt, a, e, tid);
-    tc_stage_async(raw, fv, nxt, a, tid, sbar_a);
-    if (e + 1 < e_end) tc_load_ptrs(nxt, a, e + 1, tid);
+    TcPtrs<D> nxt;
+    float fv[S::fac_slots] = {};  // factor elements of the entry staged last
+    tc_load_ptrs<D>(nxt, a, w.e, tid);
+    const bool bulk0 = tc_stage_async<D>(raw, fv, nxt, a, tid, sbar_a);
+    if (w1.e < nb) tc_load_ptrs<D>(nxt, a, w1.e, tid);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -581,11 +633,11 @@ __global__ void __launch_bounds__(kTcThreads, SPLIT ? 5 : 8) fwd_tc_bf16_kernel(
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
     const uint32_t mbar_a = smem_u32(mbar);
     const uint32_t xs_a = smem_u32(xs), bs_a = smem_u32(bs), xl_a = smem_u32(xl), bl_a = smem_u32(bl);
+    const uint32_t leader = elect_lane();  // of each warp; warp 0's issues the MMAs
     uint32_t phase = 0, sphase = 0;
     bool failed = false;
     bool staging = true;  // a staging copy is in flight whose phase has not been waited for
     double *cur = nullptr;
-    constexpr int MAXP = 2;  // tile pairs per entry (N <= 4096)
 
     // run sum (TMEM accumulator) -> FP64 reductions into `dst`.  Fibre c of the last mode
     // holds output positions 8c + r; after an octet transpose lane l of octet o holds
@@ -594,52 +646,55 @@ __global__ void __launch_bounds__(kTcThreads, SPLIT ? 5 : 8) fwd_tc_bf16_kernel(
     auto flush = [&](double *dst) {
         if (F < 8) {  // d = 1: one fibre, its 8 values are the whole output vector
             if (warp == 0) {
-                float v0[8], v1[8];
-                tmem_ld16(tacc, v0, v1);  // warp-collective: the whole warp loads
-                tmem_wait_ld();
+                float v[2][8];
+                tmem_ld16(tacc, v[0], v[1]);  // warp-collective: the whole warp loads
+                tmem_wait_ld(v);
                 if (lane == 0)
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) red_add_f64(dst + r, (double)v0[r]);
+                    for (int r = 0; r < 8; ++r) red_add_f64(dst + r, blk_out<double>(v[0][r]));
             }
             return;
         }
 #pragma unroll
-        for (int j = 0; j < MAXP; ++j) {
-            if (j < pairs) {
-                float v0[8], v1[8];
-                tmem_ld16(tacc + lane_base + 16u * j, v0, v1);
-                tmem_wait_ld();
-                octet_transpose(v0, lane);
-                octet_transpose(v1, lane);
+        for (int j = 0; j < pairs; ++j) {
+            {
+                float v[2][8];
+                tmem_ld16(tacc + lane_base + 16u * j, v[0], v[1]);
+                tmem_wait_ld(v);
+                octet_transpose(v[0], lane);
+                octet_transpose(v[1], lane);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int t = 2 * j + h;
                     const int c0 = t * kTileRows + warp * 32 + (lane & ~7);  // first fibre of the octet
-                    if (t < a.tiles && c0 < F) {
+                    if (c0 < F) {
                         double *p = dst + 8 * c0 + (lane & 7);
 #pragma unroll
-                        for (int r = 0; r < 8; ++r) red_add_f64(p + 8 * r, (double)(h ? v1[r] : v0[r]));
+                        for (int r = 0; r < 8; ++r) red_add_f64(p + 8 * r, blk_out<double>(v[h][r]));
                     }
                 }
             }
         }
     };
 
-    for (; e < e_end; ++e) {
-        double *o = a.out[e];
+    bool ok = true;      // this warp's waits so far; the CTA agrees on it at the next barrier
+    bool bulk = bulk0;   // how the entry being computed was staged
+    for (; w.e < nb; w = w1, w1 = w.next(a)) {
+        double *o = a.out[w.e];
         cp_async_wait_all();
-        const bool staged = mbar_wait(sbar_a, sphase);  // the slot's bulk copy (or its empty phase)
-        if (__syncthreads_or(!staged)) {  // slot complete for every thread; previous MMAs done
-            if (tid == 0) atomicCAS(&g_tc_error, 0u, 1u);
-            failed = true;
-            break;
+        ok = ok && mbar_wait(sbar_a, sphase);  // the slot's bulk copy (or its empty phase)
+        ok = __all_sync(0xffffffffu, ok);
+        // a bulk copy is complete for whoever waited for it, copies by threads need a barrier;
+        // the MMAs that read the operands are done for every thread (each waited for them)
+        if (!bulk) __syncthreads();
+        if (ok) {
+            sphase ^= 1u;
+            staging = false;
         }
-        sphase ^= 1u;
-        staging = false;
         // factor operands: B_i[n][k] = A_i(n, k) in the upper-left and lower-right blocks
 #pragma unroll
-        for (int s = 0; s < kTcFacSlots; ++s) {
-            const int v = tid + s * kTcThreads;
+        for (int s = 0; s < S::fac_slots; ++s) {
+            const int v = tid + s * S::threads;
             if (v < d * 64) {
                 const int i = v >> 6, r = v & 7, k = (v >> 3) & 7;
                 put<KIND_BF16>(bs + (size_t)i * kBf16B, r, k, fv[s]);
@@ -663,7 +718,8 @@ __global__ void __launch_bounds__(kTcThreads, SPLIT ? 5 : 8) fwd_tc_bf16_kernel(
             }
         } else {
             const uint32_t fsh = 3u * (uint32_t)(d - 1);
-            for (int q = tid; q < N / 8; q += kTcThreads) {
+#pragma unroll
+            for (int q = tid; q < N / 8; q += S::threads) {
                 // the two 16-byte halves in an order that keeps each 8-lane phase of the
                 // 16-byte loads on 8 distinct bank slots
                 const int h = (q >> 2) & 1;
@@ -685,81 +741,82 @@ __global__ void __launch_bounds__(kTcThreads, SPLIT ? 5 : 8) fwd_tc_bf16_kernel(
         }
         // the run continues when this entry adds into the same output as the previous one;
         // otherwise the previous run's sum leaves TMEM before the last mode overwrites it
-        const bool cont = (o == cur);
-        if (!cont && cur != nullptr) flush(cur);
+        const bool cont = o == cur && w.left < a.entries_per_chunk;
+        if (!cont && cur != nullptr && ok) flush(cur);
         cur = o;
         fence_async_smem();  // the staging slot has been read (generic proxy) before the bulk copy refills it
         tc_fence_before();
-        __syncthreads();
-        if (e + 1 < e_end) {
-            tc_stage_async(raw, fv, nxt, a, tid, sbar_a);
+        if (__syncthreads_or(!ok)) {
+            failed = true;
+            break;
+        }
+        if (w1.e < nb) {
+            bulk = tc_stage_async<D>(raw, fv, nxt, a, tid, sbar_a);
             staging = true;
-            if (e + 2 < e_end) tc_load_ptrs(nxt, a, e + 2, tid);
+            const TcWalk w2 = w1.next(a);
+            if (w2.e < nb) tc_load_ptrs<D>(nxt, a, w2.e, tid);
         }
 
         for (int i = 0; i < d; ++i) {  // modes 0, 1, ..., d-1
             const bool last = i == d - 1;
-            if (tid == 0) {
+            if (warp == 0) {
                 tc_fence_after();
                 const uint32_t dst = last ? tacc : tmem;
                 const uint32_t accumulate = (last && cont) ? 1u : 0u;
+#pragma unroll
                 for (int j = 0; j < pairs; ++j) {
-                    mma_bf16_mn(dst + 16u * (uint32_t)j, smem_desc(xs_a + j * kPairBytes, kMnLbo, kMnSbo),
-                                smem_desc(bs_a + i * kBf16B), accumulate);
+                    const uint32_t dj = dst + 16u * (uint32_t)j;
+                    const uint64_t xh = smem_desc(xs_a + j * kPairBytes, kMnLbo, kMnSbo), bh = smem_desc(bs_a + i * kBf16B);
+                    mma<KIND_BF16>(leader, dj, xh, bh, accumulate);
                     if constexpr (SPLIT) {
-                        mma_bf16_mn(dst + 16u * (uint32_t)j, smem_desc(xl_a + j * kPairBytes, kMnLbo, kMnSbo),
-                                    smem_desc(bs_a + i * kBf16B), 1u);
-                        mma_bf16_mn(dst + 16u * (uint32_t)j, smem_desc(xs_a + j * kPairBytes, kMnLbo, kMnSbo),
-                                    smem_desc(bl_a + i * kBf16B), 1u);
+                        mma<KIND_BF16>(leader, dj, smem_desc(xl_a + j * kPairBytes, kMnLbo, kMnSbo), bh, 1u);
+                        mma<KIND_BF16>(leader, dj, xh, smem_desc(bl_a + i * kBf16B), 1u);
                     }
                 }
-                mma_commit(mbar_a);
+                mma_commit(leader, mbar_a);
             }
-            const bool ok = mbar_wait(mbar_a, phase);
-            // the decision to leave must be uniform: the TMEM loads below are warp-collective
-            if (__syncthreads_or(!ok)) {
-                if (tid == 0) atomicCAS(&g_tc_error, 0u, 1u);
-                failed = true;
-                break;
-            }
+            // uniform over the warp (the TMEM loads below are warp-collective), over the CTA at
+            // the next barrier
+            ok = __all_sync(0xffffffffu, mbar_wait(mbar_a, phase));
             phase ^= 1u;
             tc_fence_after();
             if (!last) {
                 // fibre c = g + F/8 * kk with kk the next mode's index (c's top digit): the 8
                 // new values become the 8 consecutive fibres 8g..8g+7 of the next operand
                 const uint32_t sh = 3u * (uint32_t)(d - 2);
+                float v[2 * pairs][8];
 #pragma unroll
-                for (int j = 0; j < MAXP; ++j) {
-                    if (j < pairs) {
-                        float v0[8], v1[8];
-                        tmem_ld16(tmem + lane_base + 16u * j, v0, v1);
-                        tmem_wait_ld();
+                for (int j = 0; j < pairs; ++j) tmem_ld16(tmem + lane_base + 16u * j, v[2 * j], v[2 * j + 1]);
+                tmem_wait_ld(v);
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int t = 2 * j + h;
-                            const int c = t * kTileRows + warp * 32 + lane;
-                            if (t < a.tiles && c < F) {
-                                const float(&v)[8] = h ? v1 : v0;
-                                const uint32_t kk = (uint32_t)c >> sh, g = (uint32_t)c & ((1u << sh) - 1u);
-                                if constexpr (SPLIT) {
-                                    uint4 hi, lo;
-                                    split_bf16x8(v, hi, lo);
-                                    *reinterpret_cast<uint4 *>(xs + mn_offset(g, kk)) = hi;
-                                    *reinterpret_cast<uint4 *>(xl + mn_offset(g, kk)) = lo;
-                                } else {
-                                    *reinterpret_cast<uint4 *>(xs + mn_offset(g, kk)) =
-                                        pack_bf16x8(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
-                                }
-                            }
+                for (int t = 0; t < tiles; ++t) {
+                    const int c = t * kTileRows + warp * 32 + lane;
+                    if (c < F) {
+                        const uint32_t kk = (uint32_t)c >> sh, g = (uint32_t)c & ((1u << sh) - 1u);
+                        if constexpr (SPLIT) {
+                            uint4 hi, lo;
+                            split_bf16x8(v[t], hi, lo);
+                            *reinterpret_cast<uint4 *>(xs + mn_offset(g, kk)) = hi;
+                            *reinterpret_cast<uint4 *>(xl + mn_offset(g, kk)) = lo;
+                        } else {
+                            *reinterpret_cast<uint4 *>(xs + mn_offset(g, kk)) =
+                                pack_bf16x8(v[t][0], v[t][1], v[t][2], v[t][3], v[t][4], v[t][5], v[t][6], v[t][7]);
                         }
                     }
                 }
                 fence_async_smem();
                 tc_fence_before();
-                __syncthreads();
+                if (__syncthreads_or(!ok)) {
+                    failed = true;
+                    break;
+                }
             }
         }
         if (failed) break;
+    }
+    if (!ok || failed) {
+        failed = true;
+        if (lane == 0) atomicCAS(&g_tc_error, 0u, 1u);
     }
     cp_async_wait_all();
     // leaving early with a bulk copy still in flight: one more bounded wait for it, so
@@ -770,7 +827,21 @@ __global__ void __launch_bounds__(kTcThreads, SPLIT ? 5 : 8) fwd_tc_bf16_kernel(
     __syncthreads();
     tc_fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(S::cols) : "memory");
+}
+
+struct TcKernel {
+    void (*fn)(const TcArgs);
+    int threads, cols;
+    size_t need;  // bytes of shared memory; 32 of them for two mbarriers and the TMEM address
+};
+template <int D> static TcKernel tc_kernel(int kind)
+{
+    using S = TcShape<D>;
+    const size_t bf16 = (size_t)S::N * 4 + 64 + 32, part = S::pairs * kPairBytes + D * kBf16B;
+    if (kind == KRONMULT_COMPUTE_BF16X3) return {fwd_tc_bf16_kernel<true, D>, S::threads, S::cols, bf16 + 2 * part};
+    if (kind == KRONMULT_COMPUTE_BF16) return {fwd_tc_bf16_kernel<false, D>, S::threads, S::cols, bf16 + part};
+    return {fwd_tc_kernel<D>, S::threads, S::cols, bf16 + (size_t)S::tiles * kTileBytes + 2 * D * kBBytes};
 }
 
 // Plans and enqueues the tensor-core forward.  Returns cudaErrorNotSupported for
@@ -778,61 +849,37 @@ __global__ void __launch_bounds__(kTcThreads, SPLIT ? 5 : 8) fwd_tc_bf16_kernel(
 int launch_tc_forward(int kind, int d, int n, const float *const *mats, int stride, const float *const *in,
                       double *const *out, long long nb, cudaStream_t st, const kronmult_tuning *tune)
 {
-    if (n != 8 || d < 1) return cudaErrorNotSupported;
-    const long long Nl = pow_ll(n, d);
-    if (Nl > 4096) return cudaErrorNotSupported;
+    if (n != 8 || d < 1 || d > 4) return cudaErrorNotSupported;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return cudaErrorInvalidDevice;
     const DeviceInfo &di = device_info(dev);
+    const TcKernel k = d == 1 ? tc_kernel<1>(kind) : d == 2 ? tc_kernel<2>(kind) : d == 3 ? tc_kernel<3>(kind) : tc_kernel<4>(kind);
     TcArgs a{};
     a.mats = mats;
     a.in = in;
     a.out = out;
     a.nb = nb;
-    a.d = d;
     a.stride = stride;
-    a.N = (int)Nl;
-    const int F = a.N / 8;
-    a.tiles = (F + kTileRows - 1) / kTileRows;
-    const int pairs = (a.tiles + 1) / 2;
-    int cols = 32;
-    while (cols < 2 * 16 * pairs) cols *= 2;  // mode output + run accumulator
-    a.tmem_cols = cols;
-    const bool split = kind == KRONMULT_COMPUTE_BF16X3;
-    const bool bf16 = kind == KRONMULT_COMPUTE_BF16 || split;
-    const size_t parts = split ? 2 : 1;
-    const size_t need = (size_t)a.N * sizeof(float) +
-                        (bf16 ? parts * pairs * kPairBytes + 64 + parts * d * kBf16B
-                              : (size_t)a.tiles * kTileBytes + 64 + (size_t)2 * d * kBBytes) +
-                        32;  // + two mbarriers and the TMEM address
     // resident CTAs per SM are limited so that their tensor-memory columns fit in 512
     // (or to tuning.ctas_per_sm when that is fewer): each CTA reserves 1/max_ctas of the
     // SM's shared memory (less the per-CTA system reservation), so at most max_ctas fit
-    int max_ctas = 512 / cols;
+    int max_ctas = 512 / k.cols;
     if (tune && tune->ctas_per_sm > 0 && tune->ctas_per_sm < max_ctas) max_ctas = tune->ctas_per_sm;
     size_t smem = (size_t)di.smem_per_sm / max_ctas - (size_t)di.smem_reserved_cta;
     smem &= ~(size_t)15;
-    if (smem < need) smem = need;
+    if (smem < k.need) smem = k.need;
     if (smem > (size_t)di.max_smem_optin) return cudaErrorNotSupported;
-    const void *fn = split  ? (const void *)fwd_tc_bf16_kernel<true>
-                     : bf16 ? (const void *)fwd_tc_bf16_kernel<false>
-                            : (const void *)fwd_tc_kernel<KIND_TF32>;
+    const void *fn = (const void *)k.fn;
     if (!ensure_smem_attr(fn, smem) || !ensure_max_carveout(fn)) return cudaErrorInvalidValue;
-    // runs of 8 consecutive entries per CTA (the fan-in of a typical output group) and as
-    // many CTAs as that gives: the hardware keeps as many resident as the shared-memory
-    // reservation above allows, and that reservation keeps their TMEM within 512 columns
+    // run sums over chunks of 8 consecutive entries (the fan-in of a typical output group);
+    // one wave of CTAs walks the chunks
     long long ept = (tune && tune->entries_per_team > 0) ? tune->entries_per_team : 8;
-    if (ept < 1) ept = 1;
     if (ept > INT_MAX) ept = INT_MAX;
-    a.entries_per_cta = (int)ept;
-    const long long grid = (nb + ept - 1) / ept;
-    if (grid > INT_MAX) return cudaErrorInvalidValue;
-    if (split)
-        fwd_tc_bf16_kernel<true><<<(unsigned)grid, kTcThreads, smem, st>>>(a);
-    else if (bf16)
-        fwd_tc_bf16_kernel<false><<<(unsigned)grid, kTcThreads, smem, st>>>(a);
-    else
-        fwd_tc_kernel<KIND_TF32><<<(unsigned)grid, kTcThreads, smem, st>>>(a);
+    a.entries_per_chunk = (int)ept;
+    long long grid = (nb + ept - 1) / ept;
+    const long long wave = (long long)di.sms * tmem_occupancy(fn, k.threads, smem, k.cols, di);
+    if (grid > wave) grid = wave;
+    k.fn<<<(unsigned)grid, k.threads, smem, st>>>(a);
     return (int)cudaGetLastError();
 }
 
