@@ -87,10 +87,11 @@ int autotune_impl(int d, int n, int dtype, int nb_sample, kronmult_tuning *best,
         fill_uniform<T><<<1024, 256, 0, st>>>(x, (size_t)nb * N, 2);
         cudaMemsetAsync(y, 0, sizeof(TO) * (size_t)n_out * N, st);
         build_tables<T, TO><<<256, 256, 0, st>>>(mats, in, out, fac, x, y, nb, d, n, N, fan);
-        // FP64 n with a tensor-path kernel: that plan is a candidate too (its own shape); FP32:
-        // the default launch, which no forced team size selects (register blocks)
-        if (sizeof(T) == 4 || dmma_has_n(n)) {
-            kronmult_tuning t{0, 0, 0, 0, sizeof(T) == 4 ? 0 : 2};
+        // the default launch, which no forced team size selects (register blocks, short FP64
+        // vectors), and the tensor path for FP64 n that have one: each has its own shape
+        for (int path = 0; path <= 2; path += 2) {
+            if (path == 2 && (sizeof(T) == 4 || !dmma_has_n(n))) continue;
+            kronmult_tuning t{0, 0, 0, 0, path};
             FwdPlan<T, TO> pl;
             if (plan_forward<T, TO>(pl, d, n, mats, n, in, out, nullptr, nb, &t) == cudaSuccess && pl.smem_path) {
                 launch_plan<T, TO>(pl, st);

@@ -6,6 +6,7 @@
 #include "block_kernels.cuh"
 #include "column_kernels.cuh"
 #include "dmma_kernels.cuh"
+#include "f64_kernels.cuh"
 #include "fwd_kernels.cuh"
 #include "pair_kernels.cuh"
 #include "kronmult_gb300.h"
@@ -524,6 +525,56 @@ bool plan_block(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning 
     }
 }
 
+// FP64 short-vector plan (fwd_f64_kernel; n^d <= 2048).  Against the kernels below it at the
+// same shapes (us there / here): d = 3, n = 4 8.6 / 3.3 at 16 entries, 11.0 / 4.1 at 1000,
+// 275 / 270 at 200000; d = 4, n = 6 38.5 / 11.2 at 16, 461 / 437 at 8192; d = 3, n = 10 468 /
+// 419 at 8192; d = 1, n = 10 426 / 94 at 200000.  (With 1024 threads for n^d up to 4096 it was
+// slower: d = 6, n = 4, 3000 entries 512 / 595.)
+template <typename T, typename TO>
+bool plan_f64(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning *tune)
+{
+    if constexpr (sizeof(T) != 8 || sizeof(TO) != 8) {
+        return false;
+    } else {
+        FwdArgs<T, TO> &a = pl.args;
+        if (tune && (tune->team_size > 0 || tune->ctas_per_sm > 0 || tune->entries_per_team > 0 ||
+                     tune->prefetch > 0 || tune->fp64_path > 1))
+            return false;
+        // 1 % slower: 202.9 / 204.6 us at 60000 entries, 270 / 274 at 8192
+        if ((a.n == 5 && a.d == 3 && a.nb > 15000) || (a.n == 9 && a.d == 3 && a.nb > 2000)) return false;
+        const F64Info f = f64_lookup(a.n, a.d);
+        if (!f.fn[2]) return false;
+        // entries per CTA: one element per thread while one wave of CTAs holds the batch, else
+        // two, else four; equally many CTAs on every SM
+        long long cap = 1;
+        const void *fn = nullptr;
+        for (int r = 0; r < 3; ++r) {
+            fn = f.fn[r];
+            if (!fn) continue;
+            cap = ((long long)f.threads << r) / a.N;
+            const size_t smem_r = (size_t)cap * f.entry_bytes;
+            if (smem_r > (size_t)di.max_smem_optin || !ensure_smem_attr(fn, smem_r)) return false;
+            if (a.nb <= (long long)di.sms * occupancy(fn, f.threads, smem_r) * cap) break;
+        }
+        const long long k = (a.nb + di.sms * cap - 1) / (di.sms * cap);
+        const long long E = (a.nb + di.sms * k - 1) / (di.sms * k);
+        const size_t smem = (size_t)E * f.entry_bytes;
+        const long long grid = (a.nb + E - 1) / E;
+        if (grid > INT_MAX || smem > (size_t)di.max_smem_optin || !ensure_smem_attr(fn, smem)) return false;
+        long long threads = (E * a.N + 31) / 32 * 32;
+        if (threads > f.threads) threads = f.threads;
+        a.teams_per_cta = (int)E;
+        a.team_size = (int)threads;
+        a.entries_per_team = 1;
+        pl.fn = fn;
+        pl.smem_path = true;
+        pl.grid = dim3((unsigned)grid);
+        pl.block = dim3((unsigned)threads);
+        pl.smem = smem;
+        return true;
+    }
+}
+
 // Checks arguments and fills a plan.  Returns cudaSuccess, cudaErrorInvalidValue,
 // or cudaErrorNotSupported (vector too long for any path without a workspace).
 template <typename T, typename TO>
@@ -568,6 +619,9 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
 
     // ---- FP32, n and d known at compile time: register blocks
     if (plan_block<T, TO>(pl, di, tune)) return cudaSuccess;
+
+    // ---- FP64, short vectors
+    if (plan_f64<T, TO>(pl, di, tune)) return cudaSuccess;
 
     // ---- register in-place shared-memory path: 2 <= n <= 8, d >= 1
     if (n >= 2 && n <= 8 && d >= 1) {
