@@ -87,11 +87,16 @@ int autotune_impl(int d, int n, int dtype, int nb_sample, kronmult_tuning *best,
         fill_uniform<T><<<1024, 256, 0, st>>>(x, (size_t)nb * N, 2);
         cudaMemsetAsync(y, 0, sizeof(TO) * (size_t)n_out * N, st);
         build_tables<T, TO><<<256, 256, 0, st>>>(mats, in, out, fac, x, y, nb, d, n, N, fan);
-        // the default launch, which no forced team size selects (register blocks, short FP64
-        // vectors), and the tensor path for FP64 n that have one: each has its own shape
+        const int F = N / n;
+        const int qcap = n <= 4 ? 8 : 4;
+        // Candidates with shapes of their own, for the (d, n) that have team sizes to choose
+        // from: the default launch (FP32 register blocks: no field set; short FP64 vectors:
+        // the kernel's threads as the team size), and for FP64 n with a tensor-path kernel
+        // (whatever n) that path.
         for (int path = 0; path <= 2; path += 2) {
-            if (path == 2 && (sizeof(T) == 4 || !dmma_has_n(n))) continue;
+            if (path == 2 ? sizeof(T) == 4 || !dmma_has_n(n) : n > 8 || F > 512LL * qcap) continue;
             kronmult_tuning t{0, 0, 0, 0, path};
+            if (sizeof(T) == 8 && path == 0 && (t.team_size = f64_lookup(n, d).threads) == 0) continue;
             FwdPlan<T, TO> pl;
             if (plan_forward<T, TO>(pl, d, n, mats, n, in, out, nullptr, nb, &t) == cudaSuccess && pl.smem_path) {
                 launch_plan<T, TO>(pl, st);
@@ -110,8 +115,6 @@ int autotune_impl(int d, int n, int dtype, int nb_sample, kronmult_tuning *best,
                 }
             }
         }
-        const int F = N / n;
-        const int qcap = n <= 4 ? 8 : 4;
         for (int ts = 8; ts <= 512 && e == cudaSuccess; ts *= 2) {
             const int q = (F + ts - 1) / ts;
             if (q > qcap) continue;

@@ -537,13 +537,16 @@ bool plan_f64(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning *t
         return false;
     } else {
         FwdArgs<T, TO> &a = pl.args;
-        if (tune && (tune->team_size > 0 || tune->ctas_per_sm > 0 || tune->entries_per_team > 0 ||
-                     tune->prefetch > 0 || tune->fp64_path > 1))
-            return false;
-        // 1 % slower: 202.9 / 204.6 us at 60000 entries, 270 / 274 at 8192
-        if ((a.n == 5 && a.d == 3 && a.nb > 15000) || (a.n == 9 && a.d == 3 && a.nb > 2000)) return false;
         const F64Info f = f64_lookup(a.n, a.d);
         if (!f.fn[2]) return false;
+        // any tuning field selects the kernels below, but for this kernel's own threads as the
+        // team size (how the autotuner names this launch) and fp64_path = 1 (the FMA pipe)
+        if (tune && ((tune->team_size > 0 && (tune->team_size != f.threads || tune->fp64_path > 0)) ||
+                     tune->ctas_per_sm > 0 || tune->entries_per_team > 0 || tune->prefetch > 0 || tune->fp64_path > 1))
+            return false;
+        // 1 % slower: 202.9 / 204.6 us at 60000 entries, 270 / 274 at 8192
+        if (!(tune && tune->team_size > 0) && ((a.n == 5 && a.d == 3 && a.nb > 15000) || (a.n == 9 && a.d == 3 && a.nb > 2000)))
+            return false;
         // entries per CTA: one element per thread while one wave of CTAs holds the batch, else
         // two, else four; equally many CTAs on every SM
         long long cap = 1;
