@@ -179,6 +179,7 @@ struct GqShape {
     GqFn fn = nullptr;
     int ts = 0, team_elems = 0, vec_pad = 0;
     int block = kGroupedBlock;  // threads per CTA: a multiple of ts
+    bool snap = false;          // the run-time-n kernel
 };
 
 // The single-call planner's choice, for one team per entry at a time: fibre mapping
@@ -194,10 +195,24 @@ int gq_shape(int d, int n, bool det, const kronmult_tuning *tune, GqShape &sh)
     const bool forced = tune && tune->team_size > 0;
     constexpr int kAlign = 16 / (int)sizeof(T);
     sh.vec_pad = round_up(N, kAlign);
-    // [vector | factors], and in the deterministic mode (n <= 8) a run accumulator of
+    // [vector | factors], and in the deterministic mode (FP32, n <= 8) a run accumulator of
     // vec_pad values at the end of the slice
-    sh.team_elems = sh.vec_pad + round_up(d * n * n, kAlign) + (det && n <= 8 ? sh.vec_pad : 0);
+    sh.team_elems = sh.vec_pad + round_up(d * n * n, kAlign) + (det && n <= 8 && sizeof(T) == 4 ? sh.vec_pad : 0);
+    if (n > 8 && !forced && fp64_mapping(tune) == 0) {  // FP64, n = 9, 10
+        int ts = 8;
+        while (ts < kGroupedBlock && (N + ts - 1) / ts > 4) ts *= 2;
+        const int per = (N + ts - 1) / ts;
+        int emax = 1;
+        while (emax < per) emax *= 2;
+        sh.fn = gq_elem_lookup<T, TO>(n, emax, det);  // null for more than 8 elements per thread
+        if (sh.fn) {
+            sh.ts = ts;
+            sh.team_elems += sh.vec_pad;
+            return cudaSuccess;
+        }
+    }
     if (n > 8) {
+        sh.snap = true;
         const int ts = elem_team_size(N, 16, forced ? tune->team_size : 0, kGroupedBlock);
         if (ts == 0) return cudaErrorNotSupported;
         const int per = (N + ts - 1) / ts;
@@ -272,7 +287,7 @@ int gq_shape(int d, int n, bool det, const kronmult_tuning *tune, GqShape &sh)
 }
 
 // Double-float shape: the single-call emulated path's team (whole fibres, at most 4
-// per thread), the slice df_entry wants plus, in deterministic mode, N FP64 run sums.
+// per thread), the slice df_entry wants.
 int gq_df_shape(int d, int n, bool det, const kronmult_tuning *tune, GqShape &sh)
 {
     const long long Nl = pow_ll(n, d);
@@ -288,7 +303,7 @@ int gq_df_shape(int d, int n, bool det, const kronmult_tuning *tune, GqShape &sh
     }
     if (!ts || ts > kGroupedBlock) return cudaErrorNotSupported;
     sh.vec_pad = round_up(N, 4);
-    sh.team_elems = df_slice_floats(d, n, sh.vec_pad) + (det ? 2 * round_up(N, 2) : 0);
+    sh.team_elems = df_slice_floats(d, n, sh.vec_pad);
     sh.fn = gq_df_lookup(n, qmax, det);
     sh.ts = ts;
     return sh.fn ? cudaSuccess : cudaErrorNotSupported;
@@ -382,24 +397,49 @@ int grouped_plan_create(GroupedPlan *&out, const kronmult_group *groups, int n_g
         kronmult_tuning tt{};
         const kronmult_tuning *tp =
             (tunings && (tunings[g].team_size > 0 || fp64_mapping(&tunings[g]))) ? &tunings[g] : nullptr;
-        if (!tp && tuning_cache_lookup(G.matrix_count, G.matrix_size, dtype, tt) && tt.team_size <= kGroupedBlock)
+        // (not the single call's short-vector launch, which names no shape of these kernels)
+        if (!tp && tuning_cache_lookup(G.matrix_count, G.matrix_size, dtype, tt) && tt.team_size <= kGroupedBlock &&
+            !(dtype == KRONMULT_DTYPE_F64 && tt.entries_per_team == 0 && tt.prefetch == 0 && tt.fp64_path == 0 &&
+              tt.team_size == f64_lookup(G.matrix_size, G.matrix_count).threads))
             tp = &tt;
         GqShape sh;
         rc = shape_for(dtype, G.matrix_count, G.matrix_size, det, tp, sh);
         if (rc != cudaSuccess) break;
-        const int teams = sh.block / sh.ts;
-        const size_t smem = (size_t)teams * sh.team_elems * elem;
+        int teams = sh.block / sh.ts;
+        size_t smem = (size_t)teams * sh.team_elems * elem;
         if (smem > (size_t)di.max_smem_optin || !ensure_smem_attr((const void *)sh.fn, smem)) {
             rc = cudaErrorNotSupported;
             break;
         }
         GqLaunch L;
         L.fn = sh.fn;
-        L.smem = smem;
         L.block = sh.block;
         int per_sm = std::max(1, occupancy((const void *)sh.fn, sh.block, smem));
         if (tunings && tunings[g].ctas_per_sm > 0) per_sm = std::min(per_sm, tunings[g].ctas_per_sm);
-        L.grid = di.sms * per_sm;
+        // FP64 batches of up to three rounds of entries: as many teams as share them equally.
+        // (A last round of few entries waits for whole chains of barriers, and claims take about
+        // 1 ns apiece: d = 2, n = 5, 200 entries 28 us with 32 teams in 4 CTAs per SM, 19 in
+        // one; d = 4, n = 4, 3000 entries 50.9 with 4 CTAs of 4 teams, 43.7 with 3.)  Entries that take less than a claim (1024
+        // operations): four per team beyond 4096 teams.
+        long long want = (long long)di.sms * per_sm * teams;
+        const bool tiny = 2.0 * G.matrix_count * G.matrix_size * pow_ll(G.matrix_size, G.matrix_count) < 1024.0;
+        if (dtype == KRONMULT_DTYPE_F64 && !(tunings && tunings[g].ctas_per_sm > 0)) {
+            const long long rounds = (G.nb_batch + want - 1) / want;
+            if (rounds <= 3) want = (G.nb_batch + rounds - 1) / rounds;
+            if (tiny) want = std::min(want, std::max(4096LL, G.nb_batch / 4LL));
+            const long long per = (want + di.sms - 1) / di.sms;  // teams per SM
+            if (per < teams) {
+                const int step = sh.ts >= 32 ? 1 : 32 / sh.ts;
+                teams = round_up((int)per, step);
+                L.block = teams * sh.ts;
+                smem = (size_t)teams * sh.team_elems * elem;
+                per_sm = 1;
+            } else {
+                per_sm = (int)std::min<long long>(per_sm, (per + teams - 1) / teams);
+            }
+        }
+        L.smem = smem;
+        L.grid = (int)std::min<long long>((long long)di.sms * per_sm, (want + teams - 1) / teams);
         GqArgs &a = L.args;
         a.mats = G.matrix_list_batched;
         a.in = G.input_batched;
@@ -416,10 +456,16 @@ int grouped_plan_create(GroupedPlan *&out, const kronmult_group *groups, int n_g
         // then evens out the tail to one entry; measured 2-6 % faster than four units per
         // team on C3's groups, where an entry is 1-15 us of FP64 work); otherwise about
         // four units per resident team (deterministic mode sums runs within a unit, and
-        // single entries measured up to 14 % slower there).
+        // single entries measured up to 14 % slower there), FP64 more of at least 8 entries:
+        // a team's last unit ends the group (d = 6, n = 3, 56340 entries: 1476 us with units
+        // of 23, 1406 with 8), at most 16 per team for the memory of the partial sums.
         const long long teams_total = (long long)L.grid * teams;
-        long long unit = (a.nb + 4 * teams_total - 1) / (4 * teams_total);
-        if (dtype != KRONMULT_DTYPE_F32 && !det) unit = 1;
+        const long long per_team = tiny && dtype == KRONMULT_DTYPE_F64 ? 2 : 4;
+        long long unit = (a.nb + per_team * teams_total - 1) / (per_team * teams_total);
+        if (dtype != KRONMULT_DTYPE_F32) {
+            const long long sixteenth = (a.nb + 16 * teams_total - 1) / (16 * teams_total);
+            unit = !det ? 1 : std::min(unit, std::max(8LL, sixteenth));
+        }
         if (tunings && tunings[g].entries_per_team > 0) unit = tunings[g].entries_per_team;
         a.unit = std::max(1LL, unit);
         a.n_units = (a.nb + a.unit - 1) / a.unit;
@@ -427,14 +473,33 @@ int grouped_plan_create(GroupedPlan *&out, const kronmult_group *groups, int n_g
             rc = cudaErrorInvalidValue;
             break;
         }
+        if (!det && dtype == KRONMULT_DTYPE_F64 && !tp &&
+            !(tunings && (tunings[g].ctas_per_sm > 0 || tunings[g].entries_per_team > 0))) {
+            FwdPlan<double, double> fp;
+            fp.args.mats = reinterpret_cast<const double *const *>(a.mats);
+            fp.args.in = reinterpret_cast<const double *const *>(a.in);
+            fp.args.out = reinterpret_cast<double *const *>(a.out);
+            fp.args.nb = a.nb;
+            fp.args.d = a.d;
+            fp.args.n = a.n;
+            fp.args.stride = a.stride;
+            fp.args.N = a.N;
+            if (a.N <= 4 * kGroupedBlock && plan_f64<double, double>(fp, di, nullptr)) {
+                L.short_fn = reinterpret_cast<void (*)(const FwdArgs<double, double>)>(const_cast<void *>(fp.fn));
+                L.short_args = fp.args;
+                L.grid = (int)fp.grid.x;
+                L.block = (int)fp.block.x;
+                L.smem = fp.smem;
+            }
+        }
         if (det) {
             L.sort_m = std::max<long long>(kSortLocal, pow2_ceil(a.nb));
-            a.snap = G.matrix_size > 8 ? 1 : 0;  // run-time n: whole segments per unit
+            a.snap = sh.snap ? 1 : 0;  // run-time n: whole segments per unit
         }
         pl->launches.push_back(L);
         pl->n_units += a.n_units;
         pl->grid_max = std::max(pl->grid_max, L.grid);
-        pl->smem_max = std::max(pl->smem_max, smem);
+        pl->smem_max = std::max(pl->smem_max, L.smem);
     }
     for (int g = 0; g < n_adj && rc == cudaSuccess; ++g) {
         const kronmult_adjoint_group &A = adj[g];
@@ -535,7 +600,10 @@ int grouped_run(const GroupedPlan *pl, cudaStream_t st)
     if (!pl->launches.empty()) e = cudaMemsetAsync(pl->counters, 0, pl->launches.size() * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     auto launch = [&](const GqLaunch &L, cudaStream_t s) {
-        L.fn<<<L.grid, L.block, L.smem, s>>>(L.args);
+        if (L.short_fn)
+            L.short_fn<<<L.grid, L.block, L.smem, s>>>(L.short_args);
+        else
+            L.fn<<<L.grid, L.block, L.smem, s>>>(L.args);
         return cudaGetLastError();
     };
     const size_t n_par = (det ? 0 : pl->launches.size()) + pl->adjoints.size();

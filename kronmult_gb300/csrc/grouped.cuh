@@ -31,7 +31,7 @@ struct GqArgs {
     void *partial;                       // deterministic mode: 2 * n_units slots of N compute-type values
     unsigned *queue;                     // this group's unit counter (zeroed per run)
     long long nb, unit, n_units;
-    int snap;  // deterministic mode, n = 9..16: units moved to segment starts instead of partial slots
+    int snap;  // deterministic mode, run-time n: units moved to segment starts instead of partial slots
     int d, n, stride, N;
     int team_size, team_elems, vec_pad;  // vec_pad: offset of the factors in a team's slice
 };
@@ -39,7 +39,7 @@ struct GqArgs {
 using GqFn = void (*)(const GqArgs);
 
 // Kernel for a group: fibre mapping (compile-time n <= 8, QMAX fibres per thread),
-// element mapping with compile-time n (FP64, EMAX outputs per thread), or element
+// element mapping with compile-time n (FP64, n <= 10, EMAX outputs per thread), or element
 // mapping with n at run time (n = 9..16).  Null when no instantiation fits.
 template <typename T, typename TO> GqFn gq_fibre_lookup(int nn, int qmax, bool det);
 template <typename T, typename TO> GqFn gq_elem_lookup(int nn, int emax, bool det);
@@ -67,6 +67,9 @@ struct GqLaunch {
     int grid = 0, block = kGroupedBlock;
     size_t smem = 0;
     GqArgs args{};
+    // FP64 atomic mode, short vectors: the single call's kernel instead (no queue)
+    void (*short_fn)(const FwdArgs<double, double>) = nullptr;
+    FwdArgs<double, double> short_args{};
     // deterministic mode: sort buffers (m = power of two >= nb entries) and the group's
     // pointer tables in sorted order, which the kernel reads
     long long sort_m = 0;

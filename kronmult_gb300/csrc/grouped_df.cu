@@ -10,7 +10,7 @@
 namespace kgb {
 
 // One team per entry at a time, whole fibres per thread (df_team), the slice laid out
-// as df_entry wants it; deterministic mode keeps its N run sums (FP64) after the slice.
+// as df_entry wants it.
 template <int NN, int QMAX, bool DET>
 __global__ void __launch_bounds__(kGroupedBlock, 3) gq_df_kernel(const GqArgs a)
 {
@@ -24,20 +24,19 @@ __global__ void __launch_bounds__(kGroupedBlock, 3) gq_df_kernel(const GqArgs a)
     float *mh = xl + a.vec_pad;
     float *ml = mh + a.d * NN2;
     int *fexp = reinterpret_cast<int *>(ml + a.d * NN2);
-    double *acc = reinterpret_cast<double *>(xh + df_slice_floats(a.d, NN, a.vec_pad));
     const double *const *mats = reinterpret_cast<const double *const *>(a.mats);
     const double *const *in = reinterpret_cast<const double *const *>(a.in);
     double *const *out = reinterpret_cast<double *const *>(a.out);
-    long long b, e;
+    long long b, e, u;
     unsigned claim = gq_first_claim(a, tm);
-    while (gq_next(a, &s_unit[tm.id], tm, claim, b, e)) {
-        long long rs = b;
+    while (gq_next(a, &s_unit[tm.id], tm, claim, b, e, u)) {
+        GqRuns runs;  // deterministic mode
+        if constexpr (DET) runs.start(a, u, b, e);
         for (long long ei = b; ei < e; ++ei) {
-            bool first, last;
-            double *part = gq_run_edges<double, DET>(a, b, e, ei, rs, first, last);
-            double *o = out[ei];
+            bool store = false;
+            double *o = DET ? runs.place(out[ei], a.N, store) : out[ei];
             df_entry<NN, QMAX>(in[ei], mats + ei * a.d, a.d, a.stride, a.N, xh, xl, mh, ml, fexp, s_red + tm.id * 32,
-                               tm, [&](int p, double v) { gq_add<double, double, DET>(o, acc, part, p, v, first, last); });
+                               tm, [&](int p, double v) { gq_add<double, double, DET>(o, nullptr, nullptr, p, v, store, false); });
         }
     }
 }
