@@ -3,6 +3,7 @@
 #include <mutex>
 #include <utility>
 #include "adj_block.cuh"
+#include "adj_f64.cuh"
 #include "adj_kernels.cuh"
 #include "fwd_launch.cuh"
 
@@ -161,6 +162,43 @@ static bool adjoint_block(AdjArgs<float> a, const DeviceInfo &di, cudaStream_t s
     return true;
 }
 
+// FP64 adjoint of short vectors where (n, d) has an instantiation; false: not launched.
+static bool adjoint_f64(AdjArgs<double> a, const DeviceInfo &di, cudaStream_t st, int &rc)
+{
+    const AdjF64Info f = adj_f64_lookup(a.n, a.d);
+    if (!f.fn[2]) return false;
+    // slower there (us, element kernels / this one): odd n with one entry per CTA leaves the
+    // contraction's lanes idle (d = 6, n = 3 627 / 655 at 8192 entries, 102 / 88 at 1000; d = 4,
+    // n = 5 559 / 584 and 87 / 79); one CTA per SM and a second, short wave (106 / 113 at 200)
+    if (((a.n == 3 && a.d == 6) || (a.n == 5 && a.d == 4)) && a.nb > 4000) return false;
+    if (a.n == 7 && a.d == 4 && a.nb > di.sms && a.nb <= 2 * di.sms) return false;
+    // entries per CTA and elements per thread as in the forward's plan_f64
+    long long cap = 1;
+    const void *fn = nullptr;
+    for (int r = 0; r < 3; ++r) {
+        if (!f.fn[r]) continue;
+        fn = f.fn[r];
+        cap = ((long long)f.threads << r) / a.N;
+        while (cap > 1 && cap * f.entry_bytes > (long long)di.max_smem_optin) --cap;
+        const size_t smem = (size_t)cap * f.entry_bytes;
+        if (smem > (size_t)di.max_smem_optin || !ensure_smem_attr(fn, smem)) return false;
+        if (a.nb <= (long long)di.sms * occupancy(fn, f.threads, smem) * cap) break;
+    }
+    const long long k = (a.nb + di.sms * cap - 1) / (di.sms * cap), E = (a.nb + di.sms * k - 1) / (di.sms * k);
+    const long long grid = (a.nb + E - 1) / E;
+    if (grid > INT_MAX) return false;
+    long long threads = (E * a.N + 31) / 32 * 32;
+    if (threads > f.threads) threads = f.threads;
+    a.teams_per_cta = (int)E;
+    const int P = a.n * a.n, R = a.N / a.n;
+    a.slices = 1;
+    while (a.slices < 16 && 2 * a.slices * E * P <= threads && R >= 16 * a.slices) a.slices *= 2;
+    auto kernel = reinterpret_cast<void (*)(const AdjArgs<double>)>(const_cast<void *>(fn));
+    kernel<<<(unsigned)grid, (unsigned)threads, (size_t)E * f.entry_bytes, st>>>(a);
+    rc = (int)cudaGetLastError();
+    return true;
+}
+
 template <typename T>
 static int adjoint_async(int d, int n, const T *const *mats, int stride, const T *const *in, const T *const *gout,
                          T *const *gin, T *const *gmats, int gstride, long long nb, cudaStream_t st,
@@ -178,22 +216,24 @@ static int adjoint_async(int d, int n, const T *const *mats, int stride, const T
     if (cudaGetDevice(&dev) != cudaSuccess) return cudaErrorInvalidDevice;
     const DeviceInfo &di = device_info(dev);
     const int N = (int)Nl, R = N / n, P = n * n;
-    if constexpr (sizeof(T) == 4) {
-        if (!(tune && (tune->team_size > 0 || tune->entries_per_team > 0 || tune->ctas_per_sm > 0))) {
-            AdjArgs<float> b{};
-            b.mats = mats;
-            b.in = in;
-            b.gout = gout;
-            b.gin = gin;
-            b.gmats = gmats;
-            b.nb = nb;
-            b.d = d;
-            b.n = n;
-            b.stride = stride;
-            b.gstride = gstride;
-            b.N = N;
-            int rc = 0;
+    if (!(tune && (tune->team_size > 0 || tune->entries_per_team > 0 || tune->ctas_per_sm > 0))) {
+        AdjArgs<T> b{};
+        b.mats = mats;
+        b.in = in;
+        b.gout = gout;
+        b.gin = gin;
+        b.gmats = gmats;
+        b.nb = nb;
+        b.d = d;
+        b.n = n;
+        b.stride = stride;
+        b.gstride = gstride;
+        b.N = N;
+        int rc = 0;
+        if constexpr (sizeof(T) == 4) {
             if (adjoint_block(b, di, st, rc)) return rc;
+        } else {
+            if (adjoint_f64(b, di, st, rc)) return rc;
         }
     }
     int ts = 0;
