@@ -22,13 +22,19 @@ from . import _lib
 from .workloads import Batch
 
 _FN = {torch.float64: "kronmult_batched_f64", torch.float32: "kronmult_batched_f32"}
+_FN_ASYNC = {dt: name + "_async" for dt, name in _FN.items()}
+_FN_ADJOINT = {torch.float64: "kronmult_batched_adjoint_f64_async", torch.float32: "kronmult_batched_adjoint_f32_async"}
+
+# torch's current stream as an integer, without the Stream object that torch.cuda.current_stream()
+# builds (2.9 us a call, as long as the launch itself; this way 0.3)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def _addr(x) -> int | None:
     if x is None:
         return None
     if isinstance(x, torch.Tensor):
-        if x.numel() > 0 and not x.is_cuda:
+        if not x.is_cuda and x.numel() > 0:
             raise ValueError("pointer arrays must be device-resident (CUDA tensors)")
         return x.data_ptr()
     return int(x)
@@ -36,7 +42,9 @@ def _addr(x) -> int | None:
 
 def _stream_handle(stream) -> int | None:
     if stream is None:
-        return torch.cuda.current_stream().cuda_stream
+        if _raw_stream is None:
+            return torch.cuda.current_stream().cuda_stream
+        return _raw_stream(torch.cuda.current_device())
     if isinstance(stream, torch.cuda.Stream):
         return stream.cuda_stream
     return int(stream)
@@ -60,7 +68,7 @@ def kronmult_batched_async(matrix_count: int, matrix_size: int, matrix_list_batc
     """Enqueue the forward on `stream` (default: torch's current stream); no synchronisation."""
     if dtype not in _FN:
         raise TypeError("kronmult_batched is defined for float64 and float32 only")
-    name = _FN[dtype] + "_async"
+    name = _FN_ASYNC[dtype]
     fn = getattr(_lib.lib(), name)
     st = fn(int(matrix_count), int(matrix_size), _addr(matrix_list_batched), int(matrix_stride),
             _addr(input_batched), _addr(output_batched), _addr(workspace_batched), int(nb_batch),
@@ -97,7 +105,7 @@ class DeviceBatch:
 
     @property
     def nb(self) -> int:
-        return int(self.inputs.shape[0])
+        return self.inputs.size(0)
 
     @property
     def N(self) -> int:
@@ -123,14 +131,14 @@ class DeviceBatch:
 
     def forward(self, stream=None, tuning=None, sync: bool = False) -> None:
         """outputs[out_index[k]] += kron(factors of set fac_index[k]) . inputs[k] for all k."""
-        dt = self.inputs.dtype
-        if self.outputs.dtype == dt:
+        dt, nb = self.inputs.dtype, self.inputs.size(0)
+        if self.outputs.dtype is dt:
             if sync:
                 kronmult_batched(self.d, self.n, self.mat_ptrs, self.stride, self.in_ptrs, self.out_ptrs,
-                                 self.ws_ptrs, self.nb, dtype=dt)
+                                 self.ws_ptrs, nb, dt)
             else:
                 kronmult_batched_async(self.d, self.n, self.mat_ptrs, self.stride, self.in_ptrs, self.out_ptrs,
-                                       self.ws_ptrs, self.nb, dtype=dt, stream=stream, tuning=tuning)
+                                       self.ws_ptrs, nb, dt, stream, tuning)
         elif dt == torch.float32 and self.outputs.dtype == torch.float64:
             forward_f32_f64out(self, compute=_lib.KRONMULT_COMPUTE_FP32, stream=stream, tuning=tuning, sync=sync)
         else:
@@ -144,12 +152,9 @@ def adjoint(b: DeviceBatch, grad_outputs: torch.Tensor, grad_inputs: torch.Tenso
         grad_factors[fac_index[k]*d + i] += dL/dA_{k,i}   (summed over entries sharing the set)
     `grad_factors` has the factors' shape (same leading dimension).  Either may be None."""
     dt = b.inputs.dtype
-    name = {torch.float64: "kronmult_batched_adjoint_f64_async",
-            torch.float32: "kronmult_batched_adjoint_f32_async"}.get(dt)
+    name = _FN_ADJOINT.get(dt)
     if name is None or b.factors.dtype != dt:
         raise TypeError("adjoint is defined for float64 and float32 batches")
-    dev = b.inputs.device
-    es = b.inputs.element_size()
     N = b.N
     gout = grad_outputs.contiguous()
     if gout.dtype != dt or gout.shape[1] != N:
@@ -162,10 +167,12 @@ def adjoint(b: DeviceBatch, grad_outputs: torch.Tensor, grad_inputs: torch.Tenso
         fn = getattr(_lib.lib(), name)
         st = fn(b.d, b.n, b.mat_ptrs.data_ptr(), b.stride, b.in_ptrs.data_ptr(), gout_ptrs.data_ptr(),
                 None if gin_ptrs is None else gin_ptrs.data_ptr(),
-                None if gmat_ptrs is None else gmat_ptrs.data_ptr(), b.stride, b.nb, _stream_handle(stream),
+                None if gmat_ptrs is None else gmat_ptrs.data_ptr(), b.stride, b.inputs.size(0), _stream_handle(stream),
                 _lib.tuning_ptr(tuning))
         _lib.check(st, name)
         return
+    dev = b.inputs.device
+    es = b.inputs.element_size()
     gout_ptrs = gout.data_ptr() + b.out_index * (N * es)
     gin_ptrs = None
     if grad_inputs is not None:
