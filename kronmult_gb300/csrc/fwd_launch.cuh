@@ -446,7 +446,7 @@ template <typename TO> inline bool block_slower(int n, int d, long long nb)
     if (n == 2 && nb < 20000) return true;              // d = 6: 3.9 / 4.9 at 6000, 10.5 / 8.9 at 30000
     if (sizeof(TO) == 4) {
         if (n == 4 && d == 6) return nb < 2500;         // 10.5 / 13.8 at 1000, 40.5 / 38.4 at 6000
-        return n == 8 && d == 4 && nb < 500;            // 4.4 / 5.2 at 48, 31.8 / 22.1 at 2500
+        return n == 8 && d == 4 && nb < 1100;           // 14.5 / 15.1 at 1000, 31.8 / 22.1 at 2500
     }
     // FP64 outputs: chunks of 6-8 entries leave a wave's last teams uneven
     if (n == 2 || (n == 4 && d == 6)) return true;      // 11.1 / 17.5 (d = 6) and 183 / 193 at 30000

@@ -176,14 +176,6 @@ __device__ __forceinline__ void gq_entry_elem(const T *const *mats, const T *con
     }
 }
 
-// Atomic mode: every entry added into its output with atomics as soon as it is
-// computed.  Deterministic mode: entries in sorted order, runs of one output summed
-// in a shared-memory accumulator (team_elems covers it) and added once.  No run sums
-// in registers: the register footprint of the single-call kernels, 3 FP64 / 4 FP32
-// CTAs of 256 threads per SM.
-// Run edges of entry ei in unit [b, e) (deterministic mode): whether it starts / ends
-// a run of equal output pointers within the unit, and the partial slot its sum goes to
-// (null: the run is a whole segment, added directly).
 // FP64, deterministic mode: where the entries of unit [b, e) are added.  The entries are sorted
 // by output, so those of the output before the unit are one run (slot 2u), those of the output
 // after it another (slot 2u + 1), and every other run is a whole segment.
@@ -207,6 +199,9 @@ struct GqRuns {
     }
 };
 
+// Run edges of entry ei in unit [b, e) (FP32, deterministic mode): whether it starts / ends
+// a run of equal output pointers within the unit, and at a run's last entry the
+// partial slot its sum goes to (null: the run is a whole segment, added directly).
 template <typename T, bool DET>
 __device__ __forceinline__ T *gq_run_edges(const GqArgs &a, long long b, long long e, long long ei, long long &rs,
                                            bool &first, bool &last)
@@ -216,8 +211,9 @@ __device__ __forceinline__ T *gq_run_edges(const GqArgs &a, long long b, long lo
         first = ei == b || k[ei - 1] != k[ei];
         last = ei + 1 == e || k[ei + 1] != k[ei];
         if (first) rs = ei;
+        if (!last) return nullptr;
         const bool from_prev = rs == b && b > 0 && k[b - 1] == k[b];
-        const bool into_next = e < a.nb && k[e] == k[ei];  // sorted: then the run reaches the unit's end
+        const bool into_next = ei + 1 == e && e < a.nb && k[e] == k[ei];
         if (!from_prev && !into_next) return nullptr;
         const long long slot = 2 * (b / a.unit) + (from_prev ? 0 : 1);
         return reinterpret_cast<T *>(a.partial) + slot * (long long)a.N;
@@ -227,6 +223,9 @@ __device__ __forceinline__ T *gq_run_edges(const GqArgs &a, long long b, long lo
     }
 }
 
+// Atomic mode: every entry added into its output with atomics as soon as it is computed.
+// Deterministic mode: entries in sorted order, summed run by run.  No run sums in registers:
+// the register footprint of the single-call kernels, 3 FP64 / 4 FP32 CTAs of 256 threads per SM.
 template <typename T, typename TO, int NN, int QMAX, bool DET>
 __global__ void __launch_bounds__(kGroupedBlock, sizeof(T) == 8 ? 3 : 4) gq_fibre_kernel(const GqArgs a)
 {
