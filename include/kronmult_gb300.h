@@ -60,7 +60,8 @@ extern "C" {
 
 /* Launch shape override used by the autotuner; zero fields mean "heuristic". */
 typedef struct kronmult_tuning {
-    int team_size;        /* threads cooperating on one entry: 8,16,...,512 */
+    int team_size;        /* threads cooperating on one entry: 8,16,...,512 (FP64, n^d <= 2048: 256, or
+                             512 above 1024, with every other field 0 is the default launch) */
     int ctas_per_sm;      /* resident CTAs per SM to size the grid for (0 = occupancy; grouped
                              plans: at most this many persistent CTAs per SM); the tensor-core
                              path reserves shared memory so that at most this many CTAs are

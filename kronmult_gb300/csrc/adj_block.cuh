@@ -13,7 +13,12 @@
 // factor gradients go to the same place; only at the end of such a run are they summed over
 // the team's threads and added to the gradients.  Shared-memory traffic per entry: 2 reads
 // and 1 write per pass on the way down and up, against 3 reads and 2 writes per mode with a
-// reduction through shared memory per mode and entry before.
+// reduction through shared memory per mode and entry in the fibre-mapped kernel.
+//
+// Measured against that kernel, 8 entries per factor set: d = 3, n = 6, 16384 entries 60 -> 31 us
+// (shared-memory pipe 50 %, issue 47 %, FMA 26 %: two rounds of entries per CTA and their chain of
+// passes); d = 4, n = 8, 3904 entries 532 -> 179 us; d = 2, n = 2, 100000 entries 31.5 -> 11.6;
+// d = 3, n = 4, 100000 entries 84 -> 46.
 #pragma once
 #include "adj_kernels.cuh"
 #include "block_kernels.cuh"

@@ -247,7 +247,8 @@ __global__ void __launch_bounds__(OCC ? 256 : 512, OCC ? 3 : 1) adj_elem_kernel(
 }
 
 // ---- fibre-mapped variant (compile-time n): each thread owns whole fibres and keeps
-// them in registers; used for FP32, where register reuse matters more than idle lanes
+// them in registers; used for FP32 beyond the register blocks' (n, d), where register reuse
+// matters more than idle lanes
 
 // forward-style mode product (contract fastest index), src -> dst (distinct buffers)
 template <typename T, int NN, int QMAX>

@@ -2,8 +2,8 @@
 //
 // For a (d, n, dtype) the tuner builds a synthetic batch on the current GPU (own
 // factors and inputs per entry, fan-in 8, inputs larger than L2), times every
-// valid candidate (team size x entries per team) with CUDA events, keeps the
-// fastest in the cache and returns it.  The forward and grouped planners use a
+// valid candidate (team size x entries per team, and the default launch) with CUDA events,
+// keeps the fastest in the cache and returns it.  The forward and grouped planners use a
 // cached shape whenever the caller passes no explicit tuning.  The cache can be
 // saved to and loaded from a text file; entries carry the SM count of the GPU
 // they were measured on and are ignored on a different one.
