@@ -21,6 +21,7 @@
 #include "df_common.cuh"
 #include "fwd_launch.cuh"
 #include "grouped.cuh"
+#include "grouped_f64.cuh"
 #include "tuning.cuh"
 
 namespace kgb {
@@ -316,6 +317,42 @@ int shape_for(int dtype, int d, int n, bool det, const kronmult_tuning *tune, Gq
                                        : gq_shape<float, float>(d, n, det, tune, sh);
 }
 
+// Deterministic FP64 groups of short vectors (gq_f64_det_kernel), if (n, d) has an instantiation.
+void gq_f64_det_plan(GqLaunch &L, const DeviceInfo &di)
+{
+    GqArgs &a = L.args;
+    const GqF64Info f = gq_f64_lookup(a.n, a.d);
+    if (!f.fn[2]) return;
+    // entries per step and elements per thread as in the single call's plan_f64
+    long long cap = 1, wave = 1;
+    GqFn fn = nullptr;
+    for (int r = 0; r < 3; ++r) {
+        if (!f.fn[r]) continue;
+        fn = f.fn[r];
+        cap = ((long long)f.threads << r) / a.N;
+        const size_t smem = (size_t)cap * f.entry_bytes;
+        if (smem > (size_t)di.max_smem_optin || !ensure_smem_attr((const void *)fn, smem)) return;
+        wave = (long long)di.sms * std::max(1, occupancy((const void *)fn, f.threads, smem));
+        if (a.nb <= wave * cap) break;
+    }
+    const long long k = (a.nb + di.sms * cap - 1) / (di.sms * cap), E = (a.nb + di.sms * k - 1) / (di.sms * k);
+    // units of at least 8 entries (runs that cross unit edges go through memory twice: d = 6,
+    // n = 3, 56340 entries 1422 us with units of 2, 1381 of 4, 1367 of 8, 1353 of 12, 1394 of 16)
+    // where four waves of them remain, and at most 32768 units for the memory of the partial sums
+    long long least = a.nb / 32768;
+    if (a.nb / 8 >= 4 * wave) least = std::max(least, 8LL);
+    const long long unit = E * std::max(1LL, (least + E - 1) / E);
+    const long long n_units = (a.nb + unit - 1) / unit;
+    if (n_units > INT_MAX) return;
+    a.team_elems = (int)E;
+    a.unit = unit;
+    a.n_units = n_units;
+    L.fn = fn;
+    L.grid = (int)n_units;
+    L.block = (int)std::min<long long>((E * a.N + 31) / 32 * 32, f.threads);
+    L.smem = (size_t)E * f.entry_bytes;
+}
+
 long long pow2_ceil(long long v)
 {
     long long p = 1;
@@ -492,9 +529,12 @@ int grouped_plan_create(GroupedPlan *&out, const kronmult_group *groups, int n_g
                 L.smem = fp.smem;
             }
         }
+        if (det && dtype == KRONMULT_DTYPE_F64 && !tp &&
+            !(tunings && (tunings[g].ctas_per_sm > 0 || tunings[g].entries_per_team > 0)))
+            gq_f64_det_plan(L, di);
         if (det) {
             L.sort_m = std::max<long long>(kSortLocal, pow2_ceil(a.nb));
-            a.snap = sh.snap ? 1 : 0;  // run-time n: whole segments per unit
+            a.snap = sh.snap && L.fn == sh.fn ? 1 : 0;  // run-time n: whole segments per unit
         }
         pl->launches.push_back(L);
         pl->n_units += a.n_units;
