@@ -53,7 +53,7 @@ template <int NN_, int D_, int M_, int G_, int GB_, int W_, int C_, int CTAS_> s
 template <int NN, int D> struct BlkLarge;
 template <int D> struct BlkLarge<2, D> : BlkCfg<2, D, (D <= 5 ? 3 : 4), 1, (D <= 5 ? 4 : 8), 1, 4, 8> {};
 template <int D> struct BlkLarge<3, D> : BlkCfg<3, D, (D >= 5 ? 3 : 2), (D == 6 ? 2 : 1), (D >= 5 ? 9 : 3), 1, 4, (D == 6 ? 3 : D >= 7 ? 4 : D == 5 ? 5 : 8)> {};
-template <int D> struct BlkLarge<4, D> : BlkCfg<4, D, (D >= 5 ? 3 : D == 2 ? 1 : 2), 1, (D >= 5 ? 16 : D == 2 ? 1 : 4), 1, (D == 6 ? 2 : 4), (D == 6 ? 6 : D >= 5 ? 3 : 8)> {};
+template <int D> struct BlkLarge<4, D> : BlkCfg<4, D, (D >= 5 ? 3 : D == 2 ? 1 : 2), 1, (D == 6 ? 8 : D >= 5 ? 16 : D == 2 ? 1 : 4), 1, (D == 6 ? 2 : 4), (D == 6 ? 6 : D >= 5 ? 3 : 8)> {};
 template <int D> struct BlkLarge<5, D> : BlkCfg<5, D, (D == 2 ? 1 : 2), (D == 5 ? 2 : 1), (D == 2 ? 1 : 5), 1, 4, (D == 2 ? 8 : D == 3 ? 4 : D == 4 ? 5 : 3)> {};
 template <int D> struct BlkLarge<6, D> : BlkCfg<6, D, (D == 2 ? 1 : 2), 1, (D == 2 ? 1 : 6), (D >= 4 ? 8 : 1), (D >= 4 ? 1 : 4), (D >= 4 ? 2 : D == 2 ? 8 : 4)> {};
 template <int D> struct BlkLarge<7, D> : BlkCfg<7, D, (D == 2 ? 1 : 2), 1, (D == 2 ? 1 : 7), (D == 4 ? 8 : 1), (D == 4 ? 1 : 4), (D == 4 ? 2 : D == 2 ? 8 : 4)> {};
@@ -149,8 +149,13 @@ __device__ __forceinline__ void blk_mode(X (&x)[NX], unsigned fac)
                 if (f < NF) {
                     const X xk = x[f / ST * ST * NN + f % ST + k * ST];
 #pragma unroll
-                    for (int r = 0; r < NN; ++r)
+                    for (int rr = 0; rr < NN; ++rr) {
+                        // there and back: the factor value at a turn meets two values in a row
+                        // (fewer register-port conflicts: d = 3, n = 6 106 -> 100 us, d = 4,
+                        // n = 8 103 -> 101, no shape slower)
+                        const int r = g % 2 ? NN - 1 - rr : rr;
                         y[g][r] = blk_fma(m[k * NN + r], xk, k == 0 ? blk_zero(xk) : y[g][r]);
+                    }
                 }
             }
         }
