@@ -11,7 +11,7 @@
 // memory until the output or the tile changes.
 //
 // Against one mode per shared-memory round trip in both passes (split_kernels.cuh): n = 8,
-// d = 6, 3905 entries 4954 -> 2806 us, 20 -> 35 TFLOP/s; pass 1 takes two thirds of it.
+// d = 6, 3905 entries 4954 -> 2746 us, 20 -> 36 TFLOP/s; pass 1 takes two thirds of it.
 // Neither pass is at a limit of the memory (4.2-4.5 TB/s, workspace included) or of the FMA
 // pipe (48 %): 64 values per thread leave 12 warps per SM to cover the waits for the copies,
 // the shared-memory round trips between the two parts of pass 1 and their barriers.

@@ -214,7 +214,7 @@ int tmem_occupancy(const void *fn, int block, size_t smem, int cols, const Devic
 
 // Both passes in register blocks (column_kernels.cuh), for the vectors plan_split takes and
 // pl holds its plan of.  Faster at every shape and batch measured (us, plan_split's kernels /
-// these): n = 8, d = 6 19.9 / 14.0 at 8 entries, 4954 / 2806 at 3905; n = 7, d = 6 2646 / 1507
+// these): n = 8, d = 6 19.9 / 14.0 at 8 entries, 4954 / 2746 at 3905; n = 7, d = 6 2646 / 1507
 // at 3000; n = 8, d = 5 18.0 / 13.9 at 60; n = 2, d = 16 2237 / 725 at 3500.
 template <typename T, typename TO> bool plan_columns(FwdPlan<T, TO> &pl, const DeviceInfo &di)
 {
