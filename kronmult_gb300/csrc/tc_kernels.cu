@@ -37,8 +37,8 @@
 // for BF16).  Hence d at compile time, operands that stay in uniform registers for the MMAs,
 // one barrier per mode, all TMEM loads of a mode before one wait, and exact integer
 // conversion of the sums to FP64.  FP32 storage, FP64 outputs, 32768 entries of d = 4: TF32
-// 224 -> 170 us (3.9 TB/s; shared-memory pipe 63 % busy), BF16 140 -> 128 us, split BF16 225
-// -> 201 us; 200000 entries of d = 2: TF32 349 -> 110, BF16 302 -> 111, split 466 -> 181 us.
+// 224 -> 176 us (shared-memory pipe 63 % busy), BF16 140 -> 131 us, split BF16 225 -> 209 us;
+// 100000 entries of d = 2: TF32 176 -> 51, BF16 153 -> 52, split 232 -> 92 us.
 //
 // Every wait on an mbarrier is bounded; on timeout the kernel records an error
 // code in a device word (kronmult_device_error) and leaves after freeing its
@@ -300,7 +300,8 @@ template <int D> struct TcShape {
     static constexpr int fac_slots = (D * 64 + threads - 1) / threads;  // factor elements per thread
 };
 
-// A CTA's entries: chunks of entries_per_chunk consecutive ones, gridDim.x chunks apart.
+// A CTA's entries: chunks of entries_per_chunk consecutive ones, gridDim.x chunks apart (a grid
+// of all chunks: one each).
 // Run sums end with their chunk.  (One chunk per CTA: a CTA of a kernel that allocates tensor
 // memory starts on an SM only when the one before has given up its right to, which left the
 // small vectors waiting for CTA starts.)
@@ -394,10 +395,7 @@ template <int D> __global__ void __launch_bounds__(TcShape<D>::threads, D == 4 ?
     if (w.e >= nb) return;
     TcWalk w1 = w.next(a);  // the entry staged after it
 
-    // operands zeroed once: the zero half of each B (rows 8..15 of [A^T | 0], rows 0..7 of
-    // [0 | A^T]) and, for BF16, the K 8..15 half of A stay zero
-    for (int v = tid; v < (tiles * kTileBytes + 64 + 2 * d * kBBytes) / 16; v += S::threads)
-        reinterpret_cast<int4 *>(xs)[v] = make_int4(0, 0, 0, 0);
+    // first of all: the SM's next CTA starts only when this one has given up its right to allocate
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "n"(S::cols)
@@ -415,6 +413,11 @@ template <int D> __global__ void __launch_bounds__(TcShape<D>::threads, D == 4 ?
     tc_load_ptrs<D>(nxt, a, w.e, tid);
     const bool bulk0 = tc_stage_async<D>(raw, fv, nxt, a, tid, sbar_a);
     if (w1.e < nb) tc_load_ptrs<D>(nxt, a, w1.e, tid);
+    // while the first vector is on its way: operands zeroed once, that is the zero half of each
+    // B (rows 8..15 of [A^T | 0], rows 0..7 of [0 | A^T]) and the rows beyond F
+    for (int v = tid + (F % kTileRows == 0 ? (tiles * kTileBytes + 64) / 16 : 0);
+         v < (tiles * kTileBytes + 64 + 2 * d * kBBytes) / 16; v += S::threads)
+        reinterpret_cast<int4 *>(xs)[v] = make_int4(0, 0, 0, 0);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -604,10 +607,7 @@ __global__ void __launch_bounds__(TcShape<D>::threads, D < 4 ? 16 : SPLIT ? 5 : 
     if (w.e >= nb) return;
     TcWalk w1 = w.next(a);  // the entry staged after it
 
-    // operands zeroed once: fibres beyond F, the odd K half of an unpaired tile and the
-    // off-diagonal blocks of the factor operands stay zero
-    for (int v = tid; v < (int)(kParts * pairs * kPairBytes + 64 + kParts * d * kBf16B) / 16; v += S::threads)
-        reinterpret_cast<int4 *>(xs)[v] = make_int4(0, 0, 0, 0);
+    // first of all: the SM's next CTA starts only when this one has given up its right to allocate
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "n"(S::cols)
@@ -625,6 +625,11 @@ __global__ void __launch_bounds__(TcShape<D>::threads, D < 4 ? 16 : SPLIT ? 5 : 
     tc_load_ptrs<D>(nxt, a, w.e, tid);
     const bool bulk0 = tc_stage_async<D>(raw, fv, nxt, a, tid, sbar_a);
     if (w1.e < nb) tc_load_ptrs<D>(nxt, a, w1.e, tid);
+    // while the first vector is on its way: operands zeroed once; fibres beyond F, the odd K
+    // half of an unpaired tile and the off-diagonal blocks of the factor operands stay zero
+    for (int v = tid + (F % (2 * kTileRows) == 0 ? (int)(kParts * pairs * kPairBytes + 64) / 16 : 0);
+         v < (int)(kParts * pairs * kPairBytes + 64 + kParts * d * kBf16B) / 16; v += S::threads)
+        reinterpret_cast<int4 *>(xs)[v] = make_int4(0, 0, 0, 0);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -878,7 +883,11 @@ int launch_tc_forward(int kind, int d, int n, const float *const *mats, int stri
     a.entries_per_chunk = (int)ept;
     long long grid = (nb + ept - 1) / ept;
     const long long wave = (long long)di.sms * tmem_occupancy(fn, k.threads, smem, k.cols, di);
-    if (grid > wave) grid = wave;
+    // d = 4, more than two waves: a CTA per chunk.  CTAs that walk chunks leave the order of the
+    // batch, and outputs with few entries then cost more in memory (56000 entries, TF32: 774 us
+    // in one wave, 699 with a CTA per chunk for outputs of one entry, 377 and 356 for three,
+    // 289.5 either way for eight; 8192 entries: 131 and 135, 73 and 75, 59 and 61)
+    if (grid > wave && !(d == 4 && grid > 2 * wave)) grid = wave;
     k.fn<<<(unsigned)grid, k.threads, smem, st>>>(a);
     return (int)cudaGetLastError();
 }
