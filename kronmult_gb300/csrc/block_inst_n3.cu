@@ -11,9 +11,7 @@ KGB_BLK_N(float, 3,
           KGB_BLK_D(float, 3, 7)
           KGB_BLK_D(float, 3, 8))
 KGB_BLK_N(double, 3,
-          KGB_BLK_D(double, 3, 1)
           KGB_BLK_D(double, 3, 2)
-          KGB_BLK_D(double, 3, 3)
           KGB_BLK_D(double, 3, 4)
           KGB_BLK_D(double, 3, 5)
           KGB_BLK_D(double, 3, 6)

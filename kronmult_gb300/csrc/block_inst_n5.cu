@@ -8,7 +8,6 @@ KGB_BLK_N(float, 5,
           KGB_BLK_D(float, 5, 4)
           KGB_BLK_D(float, 5, 5))
 KGB_BLK_N(double, 5,
-          KGB_BLK_D(double, 5, 1)
           KGB_BLK_D(double, 5, 2)
           KGB_BLK_D(double, 5, 3)
           KGB_BLK_D(double, 5, 4)

@@ -3,13 +3,10 @@
 namespace kgb {
 KGB_BLK_N(float, 6,
           KGB_BLK_D(float, 6, 1)
-          KGB_BLK_D(float, 6, 2)
           KGB_BLK_D(float, 6, 3)
           KGB_BLK_D(float, 6, 4)
           KGB_BLK_D(float, 6, 5))
 KGB_BLK_N(double, 6,
-          KGB_BLK_D(double, 6, 1)
-          KGB_BLK_D(double, 6, 2)
           KGB_BLK_D(double, 6, 3)
           KGB_BLK_D(double, 6, 4)
           KGB_BLK_D(double, 6, 5))

@@ -8,7 +8,6 @@ KGB_BLK_N(float, 7,
           KGB_BLK_D(float, 7, 4)
           KGB_BLK_D(float, 7, 5))
 KGB_BLK_N(double, 7,
-          KGB_BLK_D(double, 7, 1)
           KGB_BLK_D(double, 7, 2)
           KGB_BLK_D(double, 7, 3)
           KGB_BLK_D(double, 7, 4)

@@ -437,21 +437,62 @@ template <typename TO> bool block_chunks(FwdArgs<float, TO> &a, const DeviceInfo
     return true;
 }
 
-// Where the other FP32 kernels measured faster than the register blocks (us there / in
-// register blocks, at entries).
+// Where the other FP32 kernels measured faster than the register blocks: [from, to) entries.
+// Most lie where a batch is a few waves of small teams and their uneven last one costs what
+// the blocks save.  Figures: us there / in register blocks at the entries named, one output
+// per entry and (after the semicolon) one per 8 entries.  Left as they are: large batches of
+// one output per entry, whose stores the persistent teams spread over all of memory (d = 6,
+// n = 4, 30000 entries 220 / 244; FP64 outputs, d = 4, n = 8 398 / 440), where two or more
+// entries per output gain (183 / 167 and 294 / 274 at two, 171 / 155 and 247 / 221 at eight):
+// the host cannot tell them apart, and taking the entries in batch order where the outputs
+// lie apart gained 4 % there and cost 1-8 % everywhere else (registers).
+struct BlkSlower {
+    int n, d;
+    long long from, to;
+};
+constexpr BlkSlower kBlkSlowerF32[] = {
+    {2, 1, 0, 400000},     // 9.7 / 11.7 at 150000, 16.9 / 17.9; 16.0 / 15.6 at 300000
+    {2, 2, 0, 120000},     // 7.4 / 8.7; 6.8 / 7.2 at 70000, 12.8 / 12.4; 11.9 / 10.7 at 150000
+    {2, 3, 0, 50000},      // 5.9 / 6.9; 5.6 / 6.0 at 30000, 9.6 / 8.9 at 70000
+    {3, 1, 0, 50000},      // 3.5 / 4.5; 4.1 / 4.2 at 12000, 8.5 / 8.5; 8.3 / 7.6 at 70000
+    {4, 1, 0, 120000},     // 7.3 / 9.1; 7.2 / 8.1 at 70000, 12.8 / 12.8; 11.8 / 11.1 at 150000
+    {5, 1, 0, 200000},     // 9.8 / 11.2; 9.5 / 10.1 at 70000, 30.6 / 28.8; 28.9 / 22.3 at 300000
+    {6, 1, 0, 50000},      // 7.5 / 8.5; 7.4 / 7.6 at 30000, 13.2 / 11.9 at 70000
+    {3, 2, 2000, 20000},   // 4.7 / 5.2; 4.5 / 4.7 at 12000
+    {7, 2, 2000, 25000},   // 6.9 / 8.0; 6.9 / 7.8 at 12000
+    {3, 3, 2000, 20000},   // 5.1 / 6.0; 5.3 / 5.5 at 12000
+    {5, 3, 3000, 25000},   // 6.4 / 7.9; 6.4 / 7.6 at 5000
+    {6, 3, 1000, 8000},    // 6.0 / 7.6; 6.0 / 7.2 at 3000
+    {7, 3, 2500, 4000},    // 8.9 / 10.6; 8.9 / 10.2 at 3000
+    {7, 4, 0, 500},        // few threads per entry: 5.4 / 6.4 at 48
+    {8, 4, 0, 1100},       // 14.5 / 15.1 at 1000, 31.8 / 22.1 at 2500
+    {4, 6, 0, 2500},       // 10.5 / 13.8 at 1000, 40.5 / 38.4 at 6000
+};
+// FP64 outputs: chunks of 6-8 entries leave a wave's last teams uneven as well
+constexpr BlkSlower kBlkSlowerF64[] = {
+    {3, 2, 0, 200000},     // 4.6 / 5.3; 4.5 / 5.2 at 12000, 48.7 / 54.9; 45.9 / 33.5 at 300000
+    {5, 3, 3000, 40000},   // 7.3 / 8.3; 7.4 / 8.4 at 5000
+    {6, 3, 2000, 25000},   // 11.8 / 13.0; 9.4 / 10.7 at 5000
+    {7, 3, 2500, 6000},    // 9.9 / 10.8; 10.1 / 11.0 at 3000
+    {8, 3, 2500, 15000},   // 17.9 / 20.3; 15.0 / 15.9 at 5000
+    {6, 4, 0, 200},        // 5.6 / 5.9; 5.4 / 5.8 at 100
+    {7, 4, 0, 500},        // few threads per entry
+    {8, 4, 0, 4000},       // 33.4 / 37.1 at 2500, 56.3 / 53.6 at 6000
+    {4, 5, 4000, 7000},    // two entries per output, 5000: 20.8 / 24.8
+};
+// No instantiation, for the same reason: n = 6, d = 2 (39.5 / 41.7 at 200000) and, of FP64
+// outputs, d = 1 with n <= 7 (n = 7: 52.3 / 58.5; 44.4 / 39.6 at 300000, 9.0 / 9.7; 8.5 / 8.8
+// at 30000), d = 3, n = 3 (9.8 / 10.9; 9.2 / 10.0 at 30000, 86 / 104; 76 / 85 at 400000),
+// d = 6, n = 4 (183 / 193 at 30000) and n = 2.
 template <typename TO> inline bool block_slower(int n, int d, long long nb)
 {
-    if (n == 6 && d == 2) return true;                  // 39.5 / 41.7 at 200000, 8.6 / 11.8 at 30000
-    if (n == 7 && d == 4 && nb < 500) return true;      // few threads per entry: 5.4 / 6.4 at 48
-    if (n == 2 && nb < 20000) return true;              // d = 6: 3.9 / 4.9 at 6000, 10.5 / 8.9 at 30000
-    if (sizeof(TO) == 4) {
-        if (n == 4 && d == 6) return nb < 2500;         // 10.5 / 13.8 at 1000, 40.5 / 38.4 at 6000
-        return n == 8 && d == 4 && nb < 1100;           // 14.5 / 15.1 at 1000, 31.8 / 22.1 at 2500
-    }
-    // FP64 outputs: chunks of 6-8 entries leave a wave's last teams uneven
-    if (n == 2 || (n == 4 && d == 6)) return true;      // 11.1 / 17.5 (d = 6) and 183 / 193 at 30000
-    if (d == 1 && n <= 6) return true;                  // n = 6: 24.1 / 29.3 at 200000
-    return n == 8 && d == 4 && nb < 4000;               // 33.4 / 37.1 at 2500, 56.3 / 53.6 at 6000
+    auto in = [&](const auto &list) {
+        for (const BlkSlower &s : list)
+            if (s.n == n && s.d == d && nb >= s.from && nb < s.to) return true;
+        return false;
+    };
+    if (n == 2 && nb < 20000) return true;  // d = 6: 3.9 / 4.9 at 6000, 10.5 / 8.9 at 30000
+    return sizeof(TO) == 4 ? in(kBlkSlowerF32) : in(kBlkSlowerF64);
 }
 
 // FP32 register-block plan (fwd_block_kernel) where (n, d) has an instantiation.
