@@ -133,6 +133,10 @@ static bool adjoint_block(AdjArgs<float> a, const DeviceInfo &di, cudaStream_t s
 {
     const AdjBlkInfo b = adj_block_lookup(a.n, a.d);
     if (!b.fn || !ensure_max_carveout(b.fn)) return false;
+    // n = 8, d = 2: the element kernels where their grid is full (52.4 us against 60.3 here at
+    // 40000 entries, 138 against 143 at 100000; 32.7 against 28.2 at 16000, 15.1 against 7.6 at
+    // 1500)
+    if (a.n == 8 && a.d == 2 && a.nb >= 20000) return false;
     // teams per group and groups per CTA as in the forward's plan_block
     const long long spread = (long long)di.sms * 8 * 32 / b.group + 1;
     long long ew = (a.nb + spread - 1) / spread;
@@ -168,10 +172,11 @@ static bool adjoint_f64(AdjArgs<double> a, const DeviceInfo &di, cudaStream_t st
     const AdjF64Info f = adj_f64_lookup(a.n, a.d);
     if (!f.fn[2]) return false;
     // slower there (us, element kernels / this one): odd n with one entry per CTA leaves the
-    // contraction's lanes idle (d = 6, n = 3 627 / 655 at 8192 entries, 102 / 88 at 1000; d = 4,
-    // n = 5 559 / 584 and 87 / 79); one CTA per SM and a second, short wave (106 / 113 at 200)
-    if (((a.n == 3 && a.d == 6) || (a.n == 5 && a.d == 4)) && a.nb > 4000) return false;
-    if (a.n == 7 && a.d == 4 && a.nb > di.sms && a.nb <= 2 * di.sms) return false;
+    // contraction's lanes idle (d = 6, n = 3 627 / 655 at 8192 entries, 110 / 113 at 1300,
+    // 102 / 88 at 1000; d = 4, n = 5 559 / 584, 96 / 101, 87 / 79; d = 4, n = 7 516 / 557 at 1500,
+    // 310 / 279 at 700); one CTA per SM and a second, short wave (106 / 113 at 200)
+    if (((a.n == 3 && a.d == 6) || (a.n == 5 && a.d == 4)) && a.nb > 8 * di.sms) return false;
+    if (a.n == 7 && a.d == 4 && ((a.nb > di.sms && a.nb <= 2 * di.sms) || a.nb > 8 * di.sms)) return false;
     // entries per CTA and elements per thread as in the forward's plan_f64
     long long cap = 1;
     const void *fn = nullptr;
