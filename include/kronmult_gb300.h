@@ -279,6 +279,13 @@ int kronmult_device_error(int *code, int clear);
  * the context usable.  Synchronises the device.  No reference counterpart. */
 int kronmult_diag_wait_selftest(int *code);
 
+/* The (n, d) that a table of kernels compiled for one (n, d) answers with: n * 100 + d of the
+ * kernel found, 0 where the table has none.  table: 0 FP64 forward of short vectors, 1 FP64
+ * adjoint, 2 deterministic FP64 groups, 3 FP32 forward, 4 the same into FP64 outputs, 5 FP32
+ * adjoint, 6 pass 1 of FP32 vectors beyond shared memory (d: its axes); -1 for another table.
+ * On the host only, no GPU needed. */
+int kronmult_diag_compiled_shape(int table, int n, int d);
+
 /* Diagnostic: measured FP64 FMA throughput of the current GPU in GFLOP/s (no
  * reference counterpart).  Allocates and synchronises; not for use in a graph. */
 int kronmult_diag_fp64_fma_gflops(double *gflops);

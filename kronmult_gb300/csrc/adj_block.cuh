@@ -406,13 +406,14 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) adj_block_ker
 
 struct AdjBlkInfo {
     const void *fn = nullptr;
+    int n = 0, d = 0;  // of the instantiation
     int EW = 0, group = 0, groups = 0, slot_bytes = 0, scratch_bytes = 0, cols = 0;
 };
 template <typename CF> AdjBlkInfo adj_info_of()
 {
     using B = Blk<CF>;
     using AB = AdjBlk<CF>;
-    return AdjBlkInfo{(const void *)adj_block_kernel<CF>, B::EW, 32 * B::W, B::C, AB::SLOT * 4, AB::SCR * 4, AB::cols};
+    return AdjBlkInfo{(const void *)adj_block_kernel<CF>, CF::NN, CF::D, B::EW, 32 * B::W, B::C, AB::SLOT * 4, AB::SCR * 4, AB::cols};
 }
 
 // Axes per pass, fibres at once, warps per group, groups per CTA and CTAs per SM, by (n, d):

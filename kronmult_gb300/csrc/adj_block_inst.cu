@@ -5,7 +5,7 @@
 namespace kgb {
 AdjBlkInfo adj_block_lookup(int n, int d)
 {
-    if (d < 1 || d > 15) return AdjBlkInfo{};
+    if (d < 1 || d > 15) return AdjBlkInfo{};  // the keys below hold d in 4 bits
     switch (n * 16 + d) {
         KGB_D(2, 2) KGB_D(2, 3) KGB_D(2, 4) KGB_D(2, 5) KGB_D(2, 6) KGB_D(2, 7) KGB_D(2, 8)
         KGB_D(3, 2) KGB_D(3, 3) KGB_D(3, 4) KGB_D(3, 5) KGB_D(3, 6)

@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(AdjF64<NN, D>::threads, 1024 / AdjF64<NN, D>::
 
 struct AdjF64Info {
     const void *fn[3] = {};  // at most 1, 2 and 4 elements per thread (null: fewer than n^d per CTA)
+    int n = 0, d = 0;  // of the instantiation
     int threads = 0, entry_bytes = 0;
 };
 AdjF64Info adj_f64_lookup(int n, int d);  // fn[2] == nullptr where there is no instantiation

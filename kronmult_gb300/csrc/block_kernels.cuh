@@ -764,13 +764,14 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
 // per CTA (at most), shared-memory bytes per group and slot, tensor-memory columns per CTA.
 struct BlkInfo {
     const void *fn = nullptr;
+    int n = 0, d = 0;  // of the instantiation
     int EW = 0, group = 0, groups = 0, slot_bytes = 0, cols = 0;
 };
 
 template <typename TO, typename CF, bool UNITS = false> BlkInfo blk_info_of()
 {
     using B = Blk<CF>;
-    return BlkInfo{(const void *)fwd_block_kernel<TO, CF, UNITS>, B::EW, 32 * B::W, B::C, B::SLOT * 4, B::cols};
+    return BlkInfo{(const void *)fwd_block_kernel<TO, CF, UNITS>, CF::NN, CF::D, B::EW, 32 * B::W, B::C, B::SLOT * 4, B::cols};
 }
 
 // The instantiation for large batches (fn == nullptr where (n, d) has none) and, where

@@ -6,6 +6,7 @@
 #include "adj_f64.cuh"
 #include "adj_kernels.cuh"
 #include "fwd_launch.cuh"
+#include "grouped_f64.cuh"
 
 namespace kgb {
 
@@ -471,6 +472,21 @@ int kronmult_batched_adjoint_f32_async(int matrix_count, int matrix_size, const 
 long long kronmult_pow_int(int number, int power) { return pow_ll(number, power); }
 
 const char *kronmult_error_string(int status) { return cudaGetErrorString((cudaError_t)status); }
+
+int kronmult_diag_compiled_shape(int table, int n, int d)
+{
+    auto shape = [](const auto &k) { return k.n * 100 + k.d; };
+    switch (table) {
+    case 0: return shape(f64_lookup(n, d));
+    case 1: return shape(adj_f64_lookup(n, d));
+    case 2: return shape(gq_f64_lookup(n, d));
+    case 3: return shape(blk_lookup<float>(n, d).large);
+    case 4: return shape(blk_lookup<double>(n, d).large);
+    case 5: return shape(adj_block_lookup(n, d));
+    case 6: return shape(units_lookup(n, d));
+    default: return -1;
+    }
+}
 
 int kronmult_abi_version(void) { return KRONMULT_GB300_VERSION; }
 

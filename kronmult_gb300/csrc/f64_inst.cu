@@ -10,6 +10,8 @@ template <int NN, int D> static F64Info info()
     if constexpr (K::N <= K::threads) f.fn[0] = (const void *)fwd_f64_kernel<NN, D, 1>;
     if constexpr (K::N <= 2 * K::threads) f.fn[1] = (const void *)fwd_f64_kernel<NN, D, 2>;
     f.fn[2] = (const void *)fwd_f64_kernel<NN, D, 4>;
+    f.n = NN;
+    f.d = D;
     f.threads = K::threads;
     f.entry_bytes = (K::VS + K::FS) * 8;
     return f;
@@ -17,6 +19,7 @@ template <int NN, int D> static F64Info info()
 
 F64Info f64_lookup(int n, int d)
 {
+    if (d < 1 || d > 15) return F64Info{};  // the keys below hold d in 4 bits
     switch (n * 16 + d) {
     case 2 * 16 + 1: return info<2, 1>();
     case 2 * 16 + 2: return info<2, 2>();
