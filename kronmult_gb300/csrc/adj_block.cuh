@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) adj_block_ker
                             for (int j = 0; j < NV; ++j) buf[j * T + t] = v[j];
                         }
                         blk_sync<W, B::C>(group);
-                        if (last) {
+                        if (last && dst != nullptr) {  // null: no gradient of this factor wanted
                             for (int j = t; j < NV; j += T) {
                                 constexpr int L = T >= 32 ? 8 : T >= 8 ? 4 : 1;  // independent partial sums
                                 float sum[L];
