@@ -286,6 +286,12 @@ int kronmult_diag_wait_selftest(int *code);
  * On the host only, no GPU needed. */
 int kronmult_diag_compiled_shape(int table, int n, int d);
 
+/* The launch shape of the FP32 adjoint's register blocks on a GPU of `sms` SMs whose CTAs may
+ * have max_smem bytes of shared memory.  shape[6]: whether it fits, groups of warps per CTA,
+ * threads, bytes, and what one group takes of each (threads, bytes).  cudaErrorNotSupported
+ * where (n, d) has no kernel.  On the host only, no GPU needed. */
+int kronmult_diag_adjoint_block_shape(int n, int d, int nb_batch, int sms, long long max_smem, long long *shape);
+
 /* Diagnostic: measured FP64 FMA throughput of the current GPU in GFLOP/s (no
  * reference counterpart).  Allocates and synchronises; not for use in a graph. */
 int kronmult_diag_fp64_fma_gflops(double *gflops);

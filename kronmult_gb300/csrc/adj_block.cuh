@@ -435,4 +435,27 @@ KGB_ADJ_TUNE(8, (D >= 3 ? 2 : 1), 4, 1, (D >= 4 ? 8 : 4), (D >= 4 ? 1 : D == 3 ?
 // fn == nullptr where (n, d) has no instantiation
 AdjBlkInfo adj_block_lookup(int n, int d);
 
+// A launch's teams per group, groups per CTA and, from these, threads and shared memory:
+// as in the forward's plan_block, with fewer groups where their shared memory (`max_smem`
+// bytes at most) asks for it.
+struct AdjBlkShape {
+    long long ew = 0;
+    int groups = 0;
+    bool fits = false;
+    int threads(const AdjBlkInfo &b) const { return groups * b.group; }
+    size_t smem(const AdjBlkInfo &b, int slots) const { return (size_t)groups * (slots * b.slot_bytes + b.scratch_bytes); }
+};
+inline AdjBlkShape adj_block_shape(const AdjBlkInfo &b, long long nb, int sms, size_t max_smem)
+{
+    AdjBlkShape s;
+    const long long spread = (long long)sms * 8 * 32 / b.group + 1;
+    s.ew = (nb + spread - 1) / spread;
+    if (s.ew > b.EW) s.ew = b.EW;
+    s.groups = b.groups;
+    while (s.groups > 1 && (long long)(s.groups / 2) * s.ew * sms >= nb) s.groups /= 2;
+    while (s.groups > 1 && s.smem(b, 1) > max_smem) s.groups /= 2;
+    s.fits = s.smem(b, 1) <= max_smem;
+    return s;
+}
+
 }  // namespace kgb

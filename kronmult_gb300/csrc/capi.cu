@@ -138,31 +138,25 @@ static bool adjoint_block(AdjArgs<float> a, const DeviceInfo &di, cudaStream_t s
     // 40000 entries, 138 against 143 at 100000; 32.7 against 28.2 at 16000, 15.1 against 7.6 at
     // 1500)
     if (a.n == 8 && a.d == 2 && a.nb >= 20000) return false;
-    // teams per group and groups per CTA as in the forward's plan_block
-    const long long spread = (long long)di.sms * 8 * 32 / b.group + 1;
-    long long ew = (a.nb + spread - 1) / spread;
-    if (ew > b.EW) ew = b.EW;
-    int groups = b.groups;
-    while (groups > 1 && (long long)(groups / 2) * ew * di.sms >= a.nb) groups /= 2;
-    const int block = groups * b.group;
-    auto smem_of = [&](int slots) { return (size_t)groups * (slots * b.slot_bytes + b.scratch_bytes); };
-    while (groups > 1 && smem_of(1) > (size_t)di.max_smem_optin) groups /= 2;
-    if (smem_of(1) > (size_t)di.max_smem_optin || !ensure_smem_attr(b.fn, smem_of(1))) return false;
-    int slots = 1, occ = tmem_occupancy(b.fn, block, smem_of(1), b.cols, di);
-    if (a.nb > (long long)di.sms * occ * groups * ew && smem_of(2) <= (size_t)di.max_smem_optin &&
-        ensure_smem_attr(b.fn, smem_of(2))) {
-        const int occ2 = tmem_occupancy(b.fn, block, smem_of(2), b.cols, di);
+    const AdjBlkShape sh = adj_block_shape(b, a.nb, di.sms, (size_t)di.max_smem_optin);
+    if (!sh.fits || !ensure_smem_attr(b.fn, sh.smem(b, 1))) return false;
+    const int block = sh.threads(b);
+    const long long per_cta = sh.groups * sh.ew;
+    int slots = 1, occ = tmem_occupancy(b.fn, block, sh.smem(b, 1), b.cols, di);
+    if (a.nb > (long long)di.sms * occ * per_cta && sh.smem(b, 2) <= (size_t)di.max_smem_optin &&
+        ensure_smem_attr(b.fn, sh.smem(b, 2))) {
+        const int occ2 = tmem_occupancy(b.fn, block, sh.smem(b, 2), b.cols, di);
         if (occ2 == occ) slots = 2;  // (d = 3, n = 6: 28 us with 3 CTAs of one slot, 32 us with 2 of two)
     }
-    long long grid = (a.nb + groups * ew - 1) / (groups * ew);
+    long long grid = (a.nb + per_cta - 1) / per_cta;
     if (grid > (long long)di.sms * occ) grid = (long long)di.sms * occ;
-    const long long teams = grid * groups * ew;
+    const long long teams = grid * per_cta;
     if (a.nb / teams >= INT_MAX) return false;
-    a.team_size = (int)ew;
+    a.team_size = (int)sh.ew;
     a.entries_per_team = (int)(a.nb / teams);
     a.slices = slots;
     auto fn = reinterpret_cast<void (*)(const AdjArgs<float>)>(const_cast<void *>(b.fn));
-    fn<<<(unsigned)grid, block, smem_of(slots), st>>>(a);
+    fn<<<(unsigned)grid, block, sh.smem(b, slots), st>>>(a);
     rc = (int)cudaGetLastError();
     return true;
 }
@@ -486,6 +480,17 @@ int kronmult_diag_compiled_shape(int table, int n, int d)
     case 6: return shape(units_lookup(n, d));
     default: return -1;
     }
+}
+
+int kronmult_diag_adjoint_block_shape(int n, int d, int nb_batch, int sms, long long max_smem, long long *shape)
+{
+    if (!shape || nb_batch < 1 || sms < 1 || max_smem < 0) return cudaErrorInvalidValue;
+    const AdjBlkInfo b = adj_block_lookup(n, d);
+    if (!b.fn) return cudaErrorNotSupported;
+    const AdjBlkShape s = adj_block_shape(b, nb_batch, sms, (size_t)max_smem);
+    const long long v[6] = {s.fits, s.groups, s.threads(b), (long long)s.smem(b, 1), b.group, b.slot_bytes + b.scratch_bytes};
+    for (int i = 0; i < 6; ++i) shape[i] = v[i];
+    return cudaSuccess;
 }
 
 int kronmult_abi_version(void) { return KRONMULT_GB300_VERSION; }
