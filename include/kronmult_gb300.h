@@ -292,6 +292,12 @@ int kronmult_diag_compiled_shape(int table, int n, int d);
  * where (n, d) has no kernel.  On the host only, no GPU needed. */
 int kronmult_diag_adjoint_block_shape(int n, int d, int nb_batch, int sms, long long max_smem, long long *shape);
 
+/* The kernel that a forward of nb_batch entries (with a workspace) launches on the current GPU:
+ * its (mangled) name, cut to len bytes with a final 0.  dtype: KRONMULT_DTYPE_F64, _F32 or
+ * _F32_F64OUT.  Plans only, launches nothing. */
+int kronmult_diag_forward_kernel(int matrix_count, int matrix_size, int dtype, int nb_batch,
+                                 const kronmult_tuning *tuning, char *name, int len);
+
 /* Diagnostic: measured FP64 FMA throughput of the current GPU in GFLOP/s (no
  * reference counterpart).  Allocates and synchronises; not for use in a graph. */
 int kronmult_diag_fp64_fma_gflops(double *gflops);

@@ -94,6 +94,7 @@ SIGNATURES = {
     "kronmult_diag_compiled_shape": (_i, [_i, _i, _i]),
     "kronmult_diag_adjoint_block_shape": (_i, [_i, _i, _i, _i, ctypes.c_longlong,
                                                ctypes.POINTER(ctypes.c_longlong)]),
+    "kronmult_diag_forward_kernel": (_i, [_i, _i, _i, _i, _TP, ctypes.c_char_p, _i]),
     "kronmult_indexed_scratch_bytes": (ctypes.c_longlong, [_i, _i]),
     "kronmult_host_device_pointer": (_i, [_vp, ctypes.POINTER(ctypes.c_void_p)]),
     "kronmult_indexed_f64_async": (_i, [_i, _i, _i, _vp, ctypes.c_longlong, _vp, _vp, ctypes.c_longlong, _vp, _vp,

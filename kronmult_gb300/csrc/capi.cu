@@ -1,4 +1,5 @@
 // C ABI of kronmult_gb300 (declarations: include/kronmult_gb300.h).
+#include <cstdio>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -118,6 +119,19 @@ int tmem_occupancy(const void *fn, int block, size_t smem, int cols, const Devic
 
 int launch_tc_forward(int kind, int d, int n, const float *const *mats, int stride, const float *const *in,
                       double *const *out, long long nb, cudaStream_t st, const kronmult_tuning *tune);
+
+template <typename T, typename TO>
+static int forward_kernel_name(int d, int n, long long nb, const kronmult_tuning *tune, char *name, int len)
+{
+    alignas(16) static const char dummy[16] = {};  // stands for tables that a plan only passes on
+    T *const *const p = reinterpret_cast<T *const *>(dummy);
+    FwdPlan<T, TO> pl;
+    int rc = plan_forward<T, TO>(pl, d, n, p, n, p, reinterpret_cast<TO *const *>(dummy), p, nb, tune);
+    const char *s = "";
+    if (rc == cudaSuccess && pl.fn) rc = (int)cudaFuncGetName(&s, pl.fn);
+    if (rc == cudaSuccess) snprintf(name, (size_t)len, "%s", s);
+    return rc;
+}
 
 template <typename T, typename TO>
 static int forward_async(int d, int n, const T *const *mats, int stride, const T *const *in, TO *const *out,
@@ -491,6 +505,19 @@ int kronmult_diag_adjoint_block_shape(int n, int d, int nb_batch, int sms, long 
     const long long v[6] = {s.fits, s.groups, s.threads(b), (long long)s.smem(b, 1), b.group, b.slot_bytes + b.scratch_bytes};
     for (int i = 0; i < 6; ++i) shape[i] = v[i];
     return cudaSuccess;
+}
+
+int kronmult_diag_forward_kernel(int matrix_count, int matrix_size, int dtype, int nb_batch,
+                                 const kronmult_tuning *tuning, char *name, int len)
+{
+    if (!name || len < 1) return cudaErrorInvalidValue;
+    if (dtype == KRONMULT_DTYPE_F64)
+        return forward_kernel_name<double, double>(matrix_count, matrix_size, nb_batch, tuning, name, len);
+    if (dtype == KRONMULT_DTYPE_F32)
+        return forward_kernel_name<float, float>(matrix_count, matrix_size, nb_batch, tuning, name, len);
+    if (dtype == KRONMULT_DTYPE_F32_F64OUT)
+        return forward_kernel_name<float, double>(matrix_count, matrix_size, nb_batch, tuning, name, len);
+    return cudaErrorInvalidValue;
 }
 
 int kronmult_abi_version(void) { return KRONMULT_GB300_VERSION; }

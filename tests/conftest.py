@@ -40,3 +40,15 @@ def cuda():
 
     kronmult_gb300.lib()
     return torch.device("cuda:0")
+
+
+def planned_kernel(d, n, dtype, nb, tuning=None):
+    """The (mangled) name of the kernel that a forward launches on the current GPU."""
+    import ctypes
+
+    from kronmult_gb300 import _lib
+
+    name = ctypes.create_string_buffer(512)
+    _lib.check(_lib.lib().kronmult_diag_forward_kernel(d, n, dtype, nb, _lib.tuning_ptr(tuning), name, 512),
+               "kronmult_diag_forward_kernel")
+    return name.value.decode()
