@@ -107,8 +107,7 @@ template <typename CF> struct AdjBlk {
     static constexpr int RBF = P <= B::V0 ? CF::NN : B::V0 / CF::NN;  // rows of a partial reduced at a time
     static constexpr int per_thread = CF::D * P;  // a thread's partials
     static constexpr int cols_used = per_thread * ((B::threads + 127) / 128);
-    static constexpr int cols = cols_used <= 32 ? 32 : cols_used <= 64 ? 64 : cols_used <= 128 ? 128
-                                                     : cols_used <= 256 ? 256 : 512;
+    static constexpr int cols = tmem_cols(cols_used);
     static_assert(CF::G == 1 && cols_used <= 512 && (B::EW == 1 || B::W == 1 || B::C == 1), "adjoint blocks");
 };
 

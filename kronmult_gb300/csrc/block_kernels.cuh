@@ -40,6 +40,9 @@
 
 namespace kgb {
 
+// tensor memory is allocated in powers of two of at least 32 columns
+constexpr int tmem_cols(int used) { return used <= 32 ? 32 : used <= 64 ? 64 : used <= 128 ? 128 : used <= 256 ? 256 : 512; }
+
 constexpr int blk_pow(int b, int e) { return e <= 0 ? 1 : b * blk_pow(b, e - 1); }
 
 // One way to run (n, d): axes per pass (M), blocks per thread (G: 1, or 2 in packed pairs),
@@ -92,11 +95,13 @@ template <typename Tn> struct Blk {
     static constexpr int FS = D * P4 / 4 % 2 == 0 ? D * P4 + 4 : D * P4;    // an entry's factors
     static constexpr int SLOT = (EW * VS + 3) / 4 * 4 + EW * FS;            // floats per staging slot of a group
     static constexpr int passes = (D + M - 1) / M;
-    // tensor-memory columns: V per group of four warps, a power of two (and at least 32)
+    // tensor-memory columns of run sums: V per group of four warps
     static constexpr int cols_used = V * ((threads + 127) / 128);
-    static constexpr int cols = cols_used <= 32 ? 32 : cols_used <= 64 ? 64 : cols_used <= 128 ? 128
-                                                     : cols_used <= 256 ? 256 : 512;
     static_assert(cols_used <= 512, "tensor memory");
+    // FP32 outputs: a second level of run sums, where all resident CTAs have room for it
+    template <typename TO>
+    static constexpr bool two_levels = sizeof(TO) == 4 && 2 * cols_used <= 512 && tmem_cols(2 * cols_used) * ctas <= 512;
+    template <typename TO> static constexpr int cols = tmem_cols(two_levels<TO> ? 2 * cols_used : cols_used);
     static_assert(C <= 15 || W == 1, "named barriers");
     static __host__ __device__ constexpr int phys(int p) { return VP == V0 ? p : p / V0 * VP + p % V0; }
     using X = std::conditional_t<G == 2, f2, float>;  // one value, or the same value of two blocks
@@ -519,9 +524,11 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
     float *base = reinterpret_cast<float *>(smem_raw) + (size_t)group * slots * B::SLOT;
 
     // `ew` teams of every group are in use; team g of all takes `share` chunks of entries,
-    // the first `more` teams one more.  FP32 outputs: a chunk is an entry.  FP64 outputs: run
-    // sums (in FP32) are cut at chunk edges, chunk_len (at most 8) entries apart.
-    constexpr bool kCuts = sizeof(TO) == 8;
+    // the first `more` teams one more.  Run sums (in FP32) are of at most chunk_len (8 or fewer)
+    // entries.  FP64 outputs: they are cut at chunk edges, so that they are fixed by the batch.
+    // FP32 outputs: a chunk is an entry; a sum of chunk_len of them is added to the output, or
+    // (kTwo) to the run's whole sum, every 8 entries of the team's share.
+    constexpr bool kCuts = sizeof(TO) == 8, kTwo = !UNITS && B::template two_levels<TO>;
     static_assert(!UNITS || (!kCuts && T >= 8), "units are stored as FP32 by large teams");
     const int ew = a.team_size;
     const long long teams = (long long)gridDim.x * (blockDim.x / (32 * W)) * ew;
@@ -535,8 +542,9 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
         return c * a.chunk_len < a.nb ? c * a.chunk_len : a.nb;
     };
     // the most entries of any team, and whether sums outlive an entry
-    const int iters = kCuts ? (share + (more > 0 ? 1 : 0)) * a.chunk_len : share + (more > 0 ? 1 : 0);
-    const bool sums = !UNITS && (kCuts ? a.chunk_len > 1 : iters > 2);
+    const int most = share + (more > 0 ? 1 : 0);
+    const int iters = kCuts ? most * a.chunk_len : most;
+    const bool sums = !UNITS && a.chunk_len > 1 && (kCuts || iters > 2);
     // The next CTA of a kernel that can allocate tensor memory starts on this SM only when
     // this one gives up its right to: at once where nothing is allocated (held to the end,
     // it left one CTA per SM: d = 4, n = 4, 5000 entries 10.0 us).
@@ -545,7 +553,7 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
         if (warp == 0) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                              (unsigned)__cvta_generic_to_shared(&s_tmem)),
-                         "n"(B::cols)
+                         "n"(B::template cols<TO>)
                          : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -618,6 +626,8 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
     };
     TO *o = count > 0 ? out_of(e0) : nullptr;
     bool fresh = true;  // the current run starts with this entry
+    int run = 0;        // entries in its sum (where chunk_len bounds them)
+    bool whole = false;  // kTwo: the run has a sum of the second level
     long long chunk = c0 + 1;  // FP64 outputs: the next chunk and, as an entry of this team, its start
     int cut = kCuts && mine ? (int)(entry_of(chunk) - e0) : 0;
     load_ptrs(0);
@@ -675,7 +685,9 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
             o = o_next;
             continue;
         }
-        bool last = active && (!sums || o_next != o);
+        bool last = active && (!sums || o_next != o || (!kCuts && !kTwo && run + 1 == a.chunk_len));
+        bool edge = false;  // sums of runs that go on are added to the second level
+        if constexpr (kTwo) edge = it % 8 == 7;
         if constexpr (kCuts) {
             if (active && it + 1 == cut) {
                 last = true;
@@ -687,6 +699,13 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             const bool mixed = __any_sync(0xffffffffu, fresh);
             blk_tm_add<V>(tmem, y, fresh, mixed);
+        }
+        if constexpr (kTwo) {
+            const bool add = active && whole && (last || edge);
+            if (__any_sync(0xffffffffu, add)) {
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                blk_tm_add<V>(tmem + B::cols_used, y, !add, true);
+            }
         }
         if constexpr (T >= 8) {
             if (last) {
@@ -723,22 +742,31 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
 #pragma unroll 1
             for (int q0 = 0; q0 < N; q0 += 32) {
                 const int q = q0 + lane;
-                unsigned long long run = 0;
-                float sum = 0.f;
+                unsigned long long at = 0;
+                float sum = 0.f, part = 0.f;
                 auto add = [&]() {
-                    if (run != 0 && q < N) atomic_add<TO>(reinterpret_cast<TO *>(run) + q, blk_out<TO>(sum));
+                    if (at != 0 && q < N) atomic_add<TO>(reinterpret_cast<TO *>(at) + q, blk_out<TO>(EW > 8 ? part + sum : sum));
                 };
 #pragma unroll 1
                 for (unsigned left = done; left != 0; left &= left - 1) {
                     const int l = __ffs(left) - 1;
                     const unsigned long long to = __shfl_sync(0xffffffffu, out, l);
                     const float v = vec[l / T * VS + __shfl_sync(0xffffffffu, sh, l) + (q < N ? B::phys(q) : 0)];
-                    if (sizeof(TO) == 4 && to == run) {
-                        sum += v;
+                    if (sizeof(TO) == 4 && to == at) {
+                        // more than 8 teams: 8 at a time (one chain over 32 of them had more error
+                        // than the kernels before: d = 2, n = 3, 27 entries per output 1.0e-7
+                        // against 0.83e-7)
+                        if (EW > 8 && l % (8 * T) == 0) {
+                            part += sum;
+                            sum = v;
+                        } else {
+                            sum += v;
+                        }
                     } else {
                         add();
-                        run = to;
+                        at = to;
                         sum = v;
+                        part = 0.f;
                     }
                 }
                 add();
@@ -746,8 +774,10 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
             if (last) o = o_next;
         }
         __syncwarp();
-        if (__any_sync(0xffffffffu, active && !last)) blk_tm_st<V>(tmem, y);
-        fresh = last;
+        if (__any_sync(0xffffffffu, active && !last)) blk_tm_st<V>(tmem + (kTwo && edge ? B::cols_used : 0), y);
+        fresh = last || edge;
+        run = last ? 0 : run + 1;
+        if constexpr (kTwo) whole = !last && (whole || edge);
     }
     if (sums) {
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -755,7 +785,7 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
         __syncthreads();
         if (warp == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem), "n"(B::cols) : "memory");
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(s_tmem), "n"(B::template cols<TO>) : "memory");
         }
     }
 }
@@ -771,7 +801,7 @@ struct BlkInfo {
 template <typename TO, typename CF, bool UNITS = false> BlkInfo blk_info_of()
 {
     using B = Blk<CF>;
-    return BlkInfo{(const void *)fwd_block_kernel<TO, CF, UNITS>, CF::NN, CF::D, B::EW, 32 * B::W, B::C, B::SLOT * 4, B::cols};
+    return BlkInfo{(const void *)fwd_block_kernel<TO, CF, UNITS>, CF::NN, CF::D, B::EW, 32 * B::W, B::C, B::SLOT * 4, B::template cols<TO>};
 }
 
 // The instantiation for large batches (fn == nullptr where (n, d) has none) and, where

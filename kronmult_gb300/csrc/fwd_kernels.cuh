@@ -39,9 +39,9 @@ template <typename T, typename TO> struct FwdArgs {
     int split_R;           // n^(d-split_d1): values sharing a fast position (stride split_C)
     int split_L;           // fast positions per pass-2 tile
     int split_ept1;        // chunks each pass-1 team sweeps (the next one copied while computing)
-    // register-block path with FP64 outputs: the chunks that bound its FP32 run sums
-    long long chunks;      // chunks of the batch
-    int chunk_len;         // entries per chunk
+    // register-block path: the chunks that bound its FP32 run sums
+    long long chunks;      // chunks of the batch (FP32 outputs: entries)
+    int chunk_len;         // entries per chunk (FP32 outputs: entries in one run sum at most)
 };
 
 // ---- helpers ---------------------------------------------------------------

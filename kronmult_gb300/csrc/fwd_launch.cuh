@@ -521,7 +521,8 @@ bool plan_block(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning 
             if (!block_chunks<TO>(a, di, tune)) return false;
         } else {
             a.chunks = a.nb;
-            a.chunk_len = 1;
+            // FP32 run sums as long as the kernels below form them
+            a.chunk_len = tune && tune->entries_per_team > 1 ? tune->entries_per_team : a.n == 4 && a.d == 6 ? 6 : 8;
         }
         // about 8 warps per SM before groups get more than one team (a group copies and adds for
         // its teams one after another; more warps cost more than they save at 5000 entries),
@@ -535,7 +536,7 @@ bool plan_block(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning 
         auto smem_of = [&](int slots) { return (size_t)groups * slots * b.slot_bytes; };
         if (smem_of(1) > (size_t)di.max_smem_optin || !ensure_smem_attr(b.fn, smem_of(1))) return false;
         int slots = 1, occ = tmem_occupancy(b.fn, block, smem_of(1), b.cols, di);
-        if (a.nb > (long long)di.sms * occ * groups * b.EW || a.chunk_len > 1) {
+        if (a.nb > (long long)di.sms * occ * groups * b.EW || (sizeof(TO) == 8 && a.chunk_len > 1)) {
             // a second slot (the next entries copied while the current ones are computed)
             // unless it halves the resident warps
             if (smem_of(2) <= (size_t)di.max_smem_optin && ensure_smem_attr(b.fn, smem_of(2))) {
@@ -552,9 +553,9 @@ bool plan_block(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning 
         else if (grid > (long long)di.sms * occ)
             grid = (long long)di.sms * occ;
         const long long teams = grid * groups * ew;
-        if (grid > INT_MAX || (a.chunks / teams + 1) * a.chunk_len > INT_MAX) return false;
-        a.team_size = (int)ew;
+        if (grid > INT_MAX || a.chunks / teams + 1 > INT_MAX / (sizeof(TO) == 8 ? a.chunk_len : 1)) return false;
         a.entries_per_team = (int)(a.chunks / teams);
+        a.team_size = (int)ew;
         a.teams_per_cta = (int)(groups * ew);
         a.prefetch = slots == 2;
         pl.fn = b.fn;
