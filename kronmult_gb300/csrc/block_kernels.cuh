@@ -101,6 +101,8 @@ template <typename Tn> struct Blk {
     // FP32 outputs: a second level of run sums, where all resident CTAs have room for it
     template <typename TO>
     static constexpr bool two_levels = sizeof(TO) == 4 && 2 * cols_used <= 512 && tmem_cols(2 * cols_used) * ctas <= 512;
+    // batches of several waves of CTAs (plan_block)
+    template <typename TO> static constexpr bool guided = sizeof(TO) == 8 ? T > 8 : T >= 8 && !two_levels<TO> && N <= 4096;
     template <typename TO> static constexpr int cols = tmem_cols(two_levels<TO> ? 2 * cols_used : cols_used);
     static_assert(C <= 15 || W == 1, "named barriers");
     static __host__ __device__ constexpr int phys(int p) { return VP == V0 ? p : p / V0 * VP + p % V0; }
@@ -524,7 +526,8 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
     float *base = reinterpret_cast<float *>(smem_raw) + (size_t)group * slots * B::SLOT;
 
     // `ew` teams of every group are in use; team g of all takes `share` chunks of entries,
-    // the first `more` teams one more.  Run sums (in FP32) are of at most chunk_len (8 or fewer)
+    // the first `more` teams one more.  (kGuided, several waves: the teams beyond the first one take
+    // a.later_share each.)  Run sums (in FP32) are of at most chunk_len (8 or fewer)
     // entries.  FP64 outputs: they are cut at chunk edges, so that they are fixed by the batch.
     // FP32 outputs: a chunk is an entry; a sum of chunk_len of them is added to the output, or
     // (kTwo) to the run's whole sum, every 8 entries of the team's share.
@@ -535,14 +538,25 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) fwd_block_ker
     const long long team0 = ((long long)blockIdx.x * (blockDim.x / (32 * W)) + group) * ew;
     const long long chunks = kCuts || UNITS ? a.chunks : a.nb;
     const int share = a.entries_per_team;
-    const long long more = chunks - share * teams;
-    auto chunk_of = [&](long long g) { return g * share + (g < more ? g : more); };
+    constexpr bool kGuided = !UNITS && B::template guided<TO>;
+    const bool waves = kGuided && a.first_ctas > 0;
+    const long long first = waves ? (long long)a.first_ctas * (blockDim.x / (32 * W)) * ew : teams;
+    const long long more = waves ? 0 : chunks - share * teams;
+    auto chunk_of = [&](long long g) {
+        if constexpr (kGuided) {
+            if (g > first) {
+                const long long c = first * share + (g - first) * a.later_share;
+                return c < chunks ? c : chunks;
+            }
+        }
+        return g * share + (g < more ? g : more);
+    };
     auto entry_of = [&](long long c) {
         if constexpr (!kCuts) return c;
         return c * a.chunk_len < a.nb ? c * a.chunk_len : a.nb;
     };
     // the most entries of any team, and whether sums outlive an entry
-    const int most = share + (more > 0 ? 1 : 0);
+    const int most = kGuided && team0 >= first ? a.later_share : share + (more > 0 ? 1 : 0);
     const int iters = kCuts ? most * a.chunk_len : most;
     const bool sums = !UNITS && a.chunk_len > 1 && (kCuts || iters > 2);
     // The next CTA of a kernel that can allocate tensor memory starts on this SM only when
@@ -796,12 +810,14 @@ struct BlkInfo {
     const void *fn = nullptr;
     int n = 0, d = 0;  // of the instantiation
     int EW = 0, group = 0, groups = 0, slot_bytes = 0, cols = 0;
+    bool guided = false;
 };
 
 template <typename TO, typename CF, bool UNITS = false> BlkInfo blk_info_of()
 {
     using B = Blk<CF>;
-    return BlkInfo{(const void *)fwd_block_kernel<TO, CF, UNITS>, CF::NN, CF::D, B::EW, 32 * B::W, B::C, B::SLOT * 4, B::template cols<TO>};
+    return BlkInfo{(const void *)fwd_block_kernel<TO, CF, UNITS>, CF::NN, CF::D, B::EW, 32 * B::W, B::C, B::SLOT * 4, B::template cols<TO>,
+                   !UNITS && B::template guided<TO>};
 }
 
 // The instantiation for large batches (fn == nullptr where (n, d) has none) and, where

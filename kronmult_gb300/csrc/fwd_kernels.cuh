@@ -42,6 +42,8 @@ template <typename T, typename TO> struct FwdArgs {
     // register-block path: the chunks that bound its FP32 run sums
     long long chunks;      // chunks of the batch (FP32 outputs: entries)
     int chunk_len;         // entries per chunk (FP32 outputs: entries in one run sum at most)
+    int first_ctas;        // of several waves: CTAs of the first one (0: one wave)
+    int later_share;       // chunks of a team of the other ones
 };
 
 // ---- helpers ---------------------------------------------------------------

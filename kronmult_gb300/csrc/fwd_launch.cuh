@@ -459,11 +459,14 @@ constexpr BlkSlower kBlkSlowerF32[] = {
     {5, 1, 0, 200000},     // 9.8 / 11.2; 9.5 / 10.1 at 70000, 30.6 / 28.8; 28.9 / 22.3 at 300000
     {6, 1, 0, 50000},      // 7.5 / 8.5; 7.4 / 7.6 at 30000, 13.2 / 11.9 at 70000
     {3, 2, 2000, 20000},   // 4.7 / 5.2; 4.5 / 4.7 at 12000
-    {7, 2, 2000, 25000},   // 6.9 / 8.0; 6.9 / 7.8 at 12000
+    {7, 2, 2000, 50000},   // 6.9 / 8.0; 6.9 / 7.8 at 12000, just beyond two waves 9.1 / 11.3; 8.9 / 10.4 at 40000
+    {2, 5, 38900, 45000},  // just beyond one wave: 7.9 / 9.9; 7.4 / 9.4 at 40000
+    {2, 6, 0, 25000},      // 6.9 / 8.2; 6.6 / 7.7 at 20000
     {3, 3, 2000, 20000},   // 5.1 / 6.0; 5.3 / 5.5 at 12000
     {5, 3, 3000, 25000},   // 6.4 / 7.9; 6.4 / 7.6 at 5000
     {6, 3, 1000, 8000},    // 6.0 / 7.6; 6.0 / 7.2 at 3000
     {7, 3, 2500, 4000},    // 8.9 / 10.6; 8.9 / 10.2 at 3000
+    {7, 3, 9700, 10800},   // just beyond one wave: 0.89 of the speed there at 10000
     {7, 4, 0, 500},        // few threads per entry: 5.4 / 6.4 at 48
     {8, 4, 0, 1100},       // 14.5 / 15.1 at 1000, 31.8 / 22.1 at 2500
     {4, 6, 0, 2500},       // 10.5 / 13.8 at 1000, 40.5 / 38.4 at 6000
@@ -472,13 +475,15 @@ constexpr BlkSlower kBlkSlowerF32[] = {
 constexpr BlkSlower kBlkSlowerF64[] = {
     {3, 2, 0, 200000},     // 4.6 / 5.3; 4.5 / 5.2 at 12000, 48.7 / 54.9; 45.9 / 33.5 at 300000
     {5, 3, 3000, 40000},   // 7.3 / 8.3; 7.4 / 8.4 at 5000
+    {5, 3, 116000, 140000},  // just beyond one wave: 0.81 of the speed; 1.03 at 120000
     {6, 3, 2000, 25000},   // 11.8 / 13.0; 9.4 / 10.7 at 5000
     {7, 3, 2500, 6000},    // 9.9 / 10.8; 10.1 / 11.0 at 3000
-    {8, 3, 2500, 15000},   // 17.9 / 20.3; 15.0 / 15.9 at 5000
+    {8, 3, 2500, 18000},   // 17.9 / 20.3; 15.0 / 15.9 at 5000
     {6, 4, 0, 200},        // 5.6 / 5.9; 5.4 / 5.8 at 100
     {7, 4, 0, 500},        // few threads per entry
     {8, 4, 0, 4000},       // 33.4 / 37.1 at 2500, 56.3 / 53.6 at 6000
-    {4, 5, 4000, 7000},    // two entries per output, 5000: 20.8 / 24.8
+    {8, 4, 7300, 9500},    // just beyond one wave: 0.84 of the speed; 0.86 at 8000
+    {4, 5, 4000, 9500},    // two entries per output, 5000: 20.8 / 24.8
 };
 // No instantiation, for the same reason: n = 6, d = 2 (39.5 / 41.7 at 200000) and, of FP64
 // outputs, d = 1 with n <= 7 (n = 7: 52.3 / 58.5; 44.4 / 39.6 at 300000, 9.0 / 9.7; 8.5 / 8.8
@@ -546,15 +551,36 @@ bool plan_block(FwdPlan<T, TO> &pl, const DeviceInfo &di, const kronmult_tuning 
             }
         }
         if (tune && tune->ctas_per_sm > 0 && tune->ctas_per_sm < occ) occ = tune->ctas_per_sm;
-        // at most one wave of CTAs, with equal shares of the chunks
-        long long grid = (a.chunks + groups * ew - 1) / (groups * ew);
-        if (tune && tune->entries_per_team > 1 && sizeof(TO) == 4)
+        // one wave of CTAs with equal shares of the chunks
+        const long long per_cta = groups * ew, wave = (long long)di.sms * occ;
+        long long grid = (a.chunks + per_cta - 1) / per_cta;
+        if (tune && tune->entries_per_team > 1 && sizeof(TO) == 4) {
             grid = (grid + tune->entries_per_team - 1) / tune->entries_per_team;
-        else if (grid > (long long)di.sms * occ)
-            grid = (long long)di.sms * occ;
-        const long long teams = grid * groups * ew;
-        if (grid > INT_MAX || a.chunks / teams + 1 > INT_MAX / (sizeof(TO) == 8 ? a.chunk_len : 1)) return false;
-        a.entries_per_team = (int)(a.chunks / teams);
+        } else if (grid > wave) {
+            // or, large vectors, of at most nine tenths of them (FP32 outputs: eight); the rest goes in
+            // small shares to CTAs that follow as SMs come free.  (One entry per output is bound by DRAM, which serves
+            // SMs unequally: d = 6, n = 4, 60000 entries 493 -> 437 us, and 311 -> 314 at eight per
+            // output, 36864 entries 306 -> 275 and 196 -> 200; FP64 outputs, d = 4, n = 8, 36864 543
+            // -> 473 and 268 -> 248.  FP32 outputs, d = 4, n = 8: from 32 entries per team on; below,
+            // 15000 entries at eight per output 59 / 63.)  Shares
+            // of whole chunks, FP32 outputs as well: their run sums are then cut where the kernels
+            // below cut them.
+            const long long teams = wave * per_cta, len = sizeof(TO) == 8 ? 1 : a.chunk_len;
+            const long long share = a.chunks * (sizeof(TO) == 8 ? 9 : 8) / (10 * teams) / len * len, rest = a.chunks - share * teams;
+            const long long least = sizeof(TO) == 4 && a.n == 8 ? 3 * len : len;
+            grid = wave;
+            if (b.guided && a.chunk_len > 1 && share >= least && !(tune && tune->ctas_per_sm > 0)) {
+                const long long rounds = (rest + teams * len - 1) / (teams * len);
+                const long long later = sizeof(TO) == 8 ? 1 : (rest + teams * rounds - 1) / (teams * rounds);
+                a.first_ctas = (int)wave;
+                a.entries_per_team = (int)share;
+                a.later_share = (int)later;
+                grid += (rest + later * per_cta - 1) / (later * per_cta);
+            }
+        }
+        const long long teams = grid * per_cta, most = a.first_ctas > 0 ? a.entries_per_team : a.chunks / teams + 1;
+        if (grid > INT_MAX || most > INT_MAX / (sizeof(TO) == 8 ? a.chunk_len : 1)) return false;
+        if (a.first_ctas == 0) a.entries_per_team = (int)(a.chunks / teams);
         a.team_size = (int)ew;
         a.teams_per_cta = (int)(groups * ew);
         a.prefetch = slots == 2;

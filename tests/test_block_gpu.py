@@ -80,3 +80,32 @@ def test_unaligned_inputs(cuda, d, n):
     assert _lib.lib().kronmult_batched_f32(b.d, b.n, db.mat_ptrs.data_ptr(), b.stride, in_ptrs.data_ptr(),
                                            db.out_ptrs.data_ptr(), None, b.nb) == 0
     assert np.array_equal(db.outputs.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("d,n,out_dtype", [(6, 4, torch.float32), (4, 8, torch.float32), (4, 8, torch.float64),
+                                           (5, 3, torch.float64)])
+def test_several_waves(cuda, d, n, out_dtype):
+    """Large vectors in more than one wave of CTAs, ragged runs, a count that no share divides: the
+    tolerance of test_ragged_runs."""
+    from kronmult_gb300 import DeviceBatch
+    from conftest import planned_kernel
+
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(31)
+    N, nb = n ** d, {(6, 4): 19013, (4, 8): 36013, (5, 3): 95013}[d, n]
+    fan = torch.randint(1, 20, (nb,), generator=gen, device=cuda)
+    fan = fan[: int((fan.cumsum(0) < nb).sum()) + 1]
+    fan[-1] -= int(fan.sum()) - nb
+    outputs = fan.numel()
+    index = torch.arange(outputs, device=cuda).repeat_interleave(fan)
+    factors = (torch.rand((outputs * d, n * n), generator=gen, device=cuda) * 2 - 1) / n ** 0.5
+    x = torch.randn((nb, N), generator=gen, device=cuda)
+    assert "fwd_block_kernel" in planned_kernel(d, n, 1 if out_dtype == torch.float32 else 2, nb)
+    db = DeviceBatch(d, n, n, factors, x, torch.zeros((outputs, N), dtype=out_dtype, device=cuda), index, index)
+    db.forward()
+    # an output's entries share their factors: K (x_1 + x_2 + ..), in 64 bits
+    want = torch.zeros((outputs, N), dtype=torch.float64, device=cuda).index_add_(0, index, x.double())
+    mats = factors.double().view(outputs, d, n, n).transpose(-1, -2)
+    for i in range(d):
+        want = torch.matmul(mats[:, i].unsqueeze(1), want.view(outputs, n ** i, n, -1)).reshape(outputs, N)
+    assert float((db.outputs.double() - want).norm() / want.norm()) <= 1.2e-6
