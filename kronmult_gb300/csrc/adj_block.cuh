@@ -278,6 +278,8 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) adj_block_ker
                 gm_next[i] = it + 1 < count ? a.gmats[(e0 + it + 1) * D + i] : nullptr;
                 if (active && gm_next[i] != gm[i]) last = true;
             }
+            // at most 32 entries in one chain of FP32 additions
+            if (it % 32 == 31) last = active;
         }
         if (slots == 2) {
             cp_async_wait_all();
@@ -343,6 +345,28 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) adj_block_ker
             if (flush) {
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 blk_sync<W, B::C>(group);  // the q buffer's last reads are done
+                // many teams of a warp whose runs end together and go to the same places: summed over
+                // the teams, as a tree, before one addition (with one each the sums in memory had
+                // 1.65 times the error at d = 2, n = 2, 100 entries per factor set, 50000 entries, and
+                // took 14.4 us, now 8.9).  Up to 8 teams add by themselves: 10 % faster at 8 entries
+                // per factor set.
+                constexpr int kSteps = W > 1 || EW < 8 ? 0 : EW > 16 ? 5 : EW > 8 ? 4 : 3;
+                bool head = true, with[kSteps + 1], merge = false;
+                if constexpr (kSteps > 0) {
+                    const int before = __shfl_up_sync(0xffffffffu, (int)last, T);  // all lanes take part
+                    head = team == 0 || !last || !before;
+#pragma unroll
+                    for (int i = 0; i < D; ++i) {
+                        const unsigned long long at = (unsigned long long)reinterpret_cast<uintptr_t>(gm[i]);
+                        const unsigned long long prev = __shfl_up_sync(0xffffffffu, at, T);
+                        head = head || prev != at;
+                    }
+                    const unsigned rest = __ballot_sync(0xffffffffu, head) >> (lane - t) >> T;  // heads of later teams
+                    const int end = rest == 0 ? EW : team + 1 + (__ffs(rest) - 1) / T;
+                    merge = __any_sync(0xffffffffu, mine && end - team >= (EW < 9 ? EW : 9));
+#pragma unroll
+                    for (int s = 0; s < kSteps; ++s) with[s] = mine && team + (1 << s) < end;
+                }
 #pragma unroll 1
                 for (int i = 0; i < D; ++i) {
                     float *dst = nullptr;  // gm[i], selected without indexing registers
@@ -362,25 +386,42 @@ __global__ void __launch_bounds__(Blk<CF>::threads, Blk<CF>::ctas) adj_block_ker
                             for (int j = 0; j < NV; ++j) buf[j * T + t] = v[j];
                         }
                         blk_sync<W, B::C>(group);
-                        if (last && dst != nullptr) {  // null: no gradient of this factor wanted
-                            for (int j = t; j < NV; j += T) {
-                                constexpr int L = T >= 32 ? 8 : T >= 8 ? 4 : 1;  // independent partial sums
-                                float sum[L];
+                        auto team_sum = [&](int j) {
+                            constexpr int L = T >= 32 ? 8 : T >= 8 ? 4 : 1;  // independent partial sums
+                            float sum[L];
 #pragma unroll
-                                for (int l = 0; l < L; ++l) sum[l] = buf[j * T + l];
+                            for (int l = 0; l < L; ++l) sum[l] = buf[j * T + l];
 #pragma unroll 1
-                                for (int h = L; h + L <= T; h += L) {
+                            for (int h = L; h + L <= T; h += L) {
 #pragma unroll
-                                    for (int l = 0; l < L; ++l) sum[l] += buf[j * T + h + l];
+                                for (int l = 0; l < L; ++l) sum[l] += buf[j * T + h + l];
+                            }
+#pragma unroll
+                            for (int l = 0; l < L; ++l)
+                                if (l < T % L) sum[l] += buf[j * T + T / L * L + l];
+#pragma unroll
+                            for (int w = L / 2; w > 0; w /= 2)
+#pragma unroll
+                                for (int l = 0; l < w; ++l) sum[l] += sum[l + w];
+                            return sum[0];
+                        };
+                        auto place = [&](int j) { return dst + (r0 + j / NN) + (size_t)(j % NN) * a.gstride; };
+                        if (!merge) {
+                            if (last && dst != nullptr) {  // null: no gradient of this factor wanted
+                                for (int j = t; j < NV; j += T) atomic_add<float>(place(j), team_sum(j));
+                            }
+                        } else {
+#pragma unroll 1
+                            for (int j0 = 0; j0 < NV; j0 += T) {
+                                const int j = j0 + t;
+                                const bool valid = last && dst != nullptr && j < NV;
+                                float sum = valid ? team_sum(j) : 0.f;
+#pragma unroll
+                                for (int s = 0; s < kSteps; ++s) {
+                                    const float other = __shfl_down_sync(0xffffffffu, sum, T << s);
+                                    if (with[s]) sum += other;
                                 }
-#pragma unroll
-                                for (int l = 0; l < L; ++l)
-                                    if (l < T % L) sum[l] += buf[j * T + T / L * L + l];
-#pragma unroll
-                                for (int w = L / 2; w > 0; w /= 2)
-#pragma unroll
-                                    for (int l = 0; l < w; ++l) sum[l] += sum[l + w];
-                                atomic_add<float>(dst + (r0 + j / NN) + (size_t)(j % NN) * a.gstride, sum[0]);
+                                if (valid && head) atomic_add<float>(place(j), sum);
                             }
                         }
                         blk_sync<W, B::C>(group);
