@@ -93,6 +93,7 @@ class DeviceBatch:
         self.fac_index = fac_index.to(device=inputs.device, dtype=torch.int64)
         self.out_index = out_index.to(device=inputs.device, dtype=torch.int64)
         self.workspace = torch.empty_like(inputs) if with_workspace else None
+        self._adj_captured = []  # adjoint tables that captured graphs read
         self.build_pointers()
 
     @classmethod
@@ -113,6 +114,7 @@ class DeviceBatch:
 
     def build_pointers(self) -> None:
         """(Re)build the device pointer arrays from the current tensors."""
+        self._adj_tables = {}  # the adjoint's, made when it is called
         dev = self.inputs.device
         fes = self.factors.element_size()
         ies = self.inputs.element_size()
@@ -155,47 +157,72 @@ def adjoint(b: DeviceBatch, grad_outputs: torch.Tensor, grad_inputs: torch.Tenso
     name = _FN_ADJOINT.get(dt)
     if name is None or b.factors.dtype != dt:
         raise TypeError("adjoint is defined for float64 and float32 batches")
-    N = b.N
-    gout = grad_outputs.contiguous()
-    if gout.dtype != dt or gout.shape[1] != N:
+    N, es = b.N, b.inputs.element_size()
+    if grad_outputs.dtype != dt or grad_outputs.shape[1] != N:
         raise ValueError("grad_outputs must be (n_out, N) of the batch dtype")
-    key = (gout.data_ptr(), None if grad_inputs is None else grad_inputs.data_ptr(),
-           None if grad_factors is None else grad_factors.data_ptr())
-    cached = getattr(b, "_adj_tables", None)
-    if cached is not None and cached[0] == key:
-        _, gout_ptrs, gin_ptrs, gmat_ptrs = cached
-        fn = getattr(_lib.lib(), name)
-        st = fn(b.d, b.n, b.mat_ptrs.data_ptr(), b.stride, b.in_ptrs.data_ptr(), gout_ptrs.data_ptr(),
-                None if gin_ptrs is None else gin_ptrs.data_ptr(),
-                None if gmat_ptrs is None else gmat_ptrs.data_ptr(), b.stride, b.inputs.size(0), _stream_handle(stream),
-                _lib.tuning_ptr(tuning))
-        _lib.check(st, name)
-        return
-    dev = b.inputs.device
-    es = b.inputs.element_size()
-    gout_ptrs = gout.data_ptr() + b.out_index * (N * es)
-    gin_ptrs = None
-    if grad_inputs is not None:
-        if grad_inputs.shape != b.inputs.shape or grad_inputs.dtype != dt or not grad_inputs.is_contiguous():
-            raise ValueError("grad_inputs must match the inputs' shape and dtype")
-        k = torch.arange(b.nb, device=dev, dtype=torch.int64)
-        gin_ptrs = grad_inputs.data_ptr() + k * (N * es)
-    gmat_ptrs = None
-    if grad_factors is not None:
-        if grad_factors.shape != b.factors.shape or grad_factors.dtype != dt or not grad_factors.is_contiguous():
-            raise ValueError("grad_factors must match the factors' shape and dtype")
-        i = torch.arange(b.d, device=dev, dtype=torch.int64)
-        blk = b.factors.shape[1]
-        gmat_ptrs = (grad_factors.data_ptr() + (b.fac_index[:, None] * b.d + i[None, :]) * (blk * es)).reshape(-1)
-    fn = getattr(_lib.lib(), name)
-    st = fn(b.d, b.n, b.mat_ptrs.data_ptr(), b.stride, b.in_ptrs.data_ptr(), gout_ptrs.data_ptr(),
-            None if gin_ptrs is None else gin_ptrs.data_ptr(), None if gmat_ptrs is None else gmat_ptrs.data_ptr(),
-            b.stride, b.nb, _stream_handle(stream), _lib.tuning_ptr(tuning))
+    if grad_inputs is not None and (grad_inputs.shape != b.inputs.shape or grad_inputs.dtype != dt
+                                    or not grad_inputs.is_contiguous()):
+        raise ValueError("grad_inputs must match the inputs' shape and dtype")
+    if grad_factors is not None and (grad_factors.shape != b.factors.shape or grad_factors.dtype != dt
+                                     or not grad_factors.is_contiguous()):
+        raise ValueError("grad_factors must match the factors' shape and dtype")
+    handle = _stream_handle(stream)
+    if stream is not None and handle != _stream_handle(None):
+        # tables and copies are made on the stream that reads them, and their memory belongs to it
+        if not isinstance(stream, torch.cuda.Stream):
+            stream = torch.cuda.ExternalStream(handle) if handle else torch.cuda.default_stream()
+        with torch.cuda.stream(stream):
+            _adjoint_on_current(b, grad_outputs, grad_inputs, grad_factors, N, es, handle, tuning, name)
+    else:
+        _adjoint_on_current(b, grad_outputs, grad_inputs, grad_factors, N, es, handle, tuning, name)
+
+
+# pointer tables kept per batch: for so many streams
+_ADJ_STREAMS = 4
+
+
+def _version(t: torch.Tensor) -> int:
+    return -1 if t.is_inference() else t._version
+
+
+def _adjoint_on_current(b: DeviceBatch, grad_outputs, grad_inputs, grad_factors, N: int, es: int, handle, tuning,
+                        name: str) -> None:
+    """adjoint() of checked arguments on torch's current stream (`handle`)."""
+    nb = b.inputs.size(0)
+    gout = grad_outputs.contiguous()
+    # what the tables are made of, beside the two index tensors
+    key = (b.inputs.shape, b.factors.shape, gout.data_ptr(), None if grad_inputs is None else grad_inputs.data_ptr(),
+           None if grad_factors is None else grad_factors.data_ptr(), _version(b.out_index), _version(b.fac_index))
+    capturing = torch.cuda.is_current_stream_capturing()
+    tables = None
+    for kept in list(b._adj_tables.values()) if capturing else (b._adj_tables.get(handle),):
+        if kept is not None and kept[0] == key and kept[1] is b.out_index and kept[2] is b.fac_index:
+            tables = kept
+    if tables is None:
+        dev = b.inputs.device
+        gout_ptrs = gout.data_ptr() + b.out_index * (N * es)
+        gin_ptrs = gmat_ptrs = None
+        if grad_inputs is not None:
+            gin_ptrs = grad_inputs.data_ptr() + torch.arange(nb, device=dev, dtype=torch.int64) * (N * es)
+        if grad_factors is not None:
+            i = torch.arange(b.d, device=dev, dtype=torch.int64)
+            blk = b.factors.shape[1]
+            gmat_ptrs = (grad_factors.data_ptr() + (b.fac_index[:, None] * b.d + i[None, :]) * (blk * es)).reshape(-1)
+        tables = (key, b.out_index, b.fac_index, gout_ptrs, gin_ptrs, gmat_ptrs)
+        if not capturing:  # tables of a captured call belong to the graph, which fills them
+            b._adj_tables.pop(handle, None)
+            while len(b._adj_tables) >= _ADJ_STREAMS:
+                b._adj_tables.pop(next(iter(b._adj_tables)))
+            b._adj_tables[handle] = tables
+    elif capturing and not any(t is tables for t in b._adj_captured):
+        b._adj_captured.append(tables)  # the graph reads them for as long as the batch lives
+    gout_ptrs, gin_ptrs, gmat_ptrs = tables[3:]
+    st = getattr(_lib.lib(), name)(
+        b.d, b.n, b.mat_ptrs.data_ptr(), b.stride, b.in_ptrs.data_ptr(), gout_ptrs.data_ptr(),
+        None if gin_ptrs is None else gin_ptrs.data_ptr(), None if gmat_ptrs is None else gmat_ptrs.data_ptr(),
+        b.stride, nb, handle, _lib.tuning_ptr(tuning))
     _lib.check(st, name)
-    # keep the pointer tables referenced by the batch (reused while the same gradient
-    # tensors are passed) so that their memory stays valid for the enqueued kernel
-    b._adj_tables = (key, gout_ptrs, gin_ptrs, gmat_ptrs)
-    b._adj_keep = gout
+    b._adj_keep = grad_outputs  # read by the enqueued kernel, on whatever stream
 
 
 def check_device_error(clear: bool = True) -> None:
