@@ -317,6 +317,11 @@ int shape_for(int dtype, int d, int n, bool det, const kronmult_tuning *tune, Gq
                                        : gq_shape<float, float>(d, n, det, tune, sh);
 }
 
+// Bytes of partial sums that a plan's deterministic groups share (the largest group's; they run one
+// after another), unless four units per resident team take more.  Larger units where a group
+// would exceed it: d = 3, n = 10, 19000 entries 300 MB with one entry per unit.
+constexpr long long kPartialBytes = 96LL << 20;
+
 // Deterministic FP64 groups of short vectors (gq_f64_det_kernel), if (n, d) has an instantiation.
 void gq_f64_det_plan(GqLaunch &L, const DeviceInfo &di)
 {
@@ -338,8 +343,9 @@ void gq_f64_det_plan(GqLaunch &L, const DeviceInfo &di)
     const long long k = (a.nb + di.sms * cap - 1) / (di.sms * cap), E = (a.nb + di.sms * k - 1) / (di.sms * k);
     // units of at least 8 entries (runs that cross unit edges go through memory twice: d = 6,
     // n = 3, 56340 entries 1422 us with units of 2, 1381 of 4, 1367 of 8, 1353 of 12, 1394 of 16)
-    // where four waves of them remain, and at most 32768 units for the memory of the partial sums
-    long long least = a.nb / 32768;
+    // where four waves of them remain, and no more units than the memory of the partial sums admits
+    const long long most = std::max(1LL, kPartialBytes / (16LL * a.N));
+    long long least = (a.nb + most - 1) / most;
     if (a.nb / 8 >= 4 * wave) least = std::max(least, 8LL);
     const long long unit = E * std::max(1LL, (least + E - 1) / E);
     const long long n_units = (a.nb + unit - 1) / unit;
@@ -495,13 +501,13 @@ int grouped_plan_create(GroupedPlan *&out, const kronmult_group *groups, int n_g
         // four units per resident team (deterministic mode sums runs within a unit, and
         // single entries measured up to 14 % slower there), FP64 more of at least 8 entries:
         // a team's last unit ends the group (d = 6, n = 3, 56340 entries: 1476 us with units
-        // of 23, 1406 with 8), at most 16 per team for the memory of the partial sums.
+        // of 23, 1406 with 8), at most 16 per team and (beyond 4) kPartialBytes of partial sums.
         const long long teams_total = (long long)L.grid * teams;
         const long long per_team = tiny && dtype == KRONMULT_DTYPE_F64 ? 2 : 4;
         long long unit = (a.nb + per_team * teams_total - 1) / (per_team * teams_total);
         if (dtype != KRONMULT_DTYPE_F32) {
-            const long long sixteenth = (a.nb + 16 * teams_total - 1) / (16 * teams_total);
-            unit = !det ? 1 : std::min(unit, std::max(8LL, sixteenth));
+            const long long most = std::max(4 * teams_total, std::min(16 * teams_total, kPartialBytes / (16LL * pow_ll(G.matrix_size, G.matrix_count))));
+            unit = !det ? 1 : std::min(unit, std::max(8LL, (a.nb + most - 1) / most));
         }
         if (tunings && tunings[g].entries_per_team > 0) unit = tunings[g].entries_per_team;
         a.unit = std::max(1LL, unit);
@@ -557,10 +563,13 @@ int grouped_plan_create(GroupedPlan *&out, const kronmult_group *groups, int n_g
     // device memory: the queue counters, then each deterministic group's sort buffers
     auto align = [](size_t v) { return (v + 255) & ~(size_t)255; };
     size_t total = align(std::max<size_t>(1, pl->launches.size()) * sizeof(unsigned));
-    for (const GqLaunch &L : pl->launches)
-        if (L.sort_m)
-            total += align((size_t)L.sort_m * 8) * 2 + align((size_t)L.args.nb * (L.args.d + 2) * 8) +
-                     (L.args.snap ? 0 : align((size_t)2 * L.args.n_units * L.args.N * acc_elem));
+    size_t partial = 0;  // of the largest group: each one's are reduced before the next group runs
+    for (const GqLaunch &L : pl->launches) {
+        if (!L.sort_m) continue;
+        total += align((size_t)L.sort_m * 8) * 2 + align((size_t)L.args.nb * (L.args.d + 2) * 8);
+        if (!L.args.snap) partial = std::max(partial, align((size_t)2 * L.args.n_units * L.args.N * acc_elem));
+    }
+    total += partial;
     if (cudaMalloc(&pl->dmem, total) != cudaSuccess) {
         cudaGetLastError();
         destroy_plan(pl);
@@ -582,10 +591,7 @@ int grouped_plan_create(GroupedPlan *&out, const kronmult_group *groups, int n_g
             L.s_in = L.s_mats + nb * L.args.d;
             L.s_out = const_cast<void **>(L.s_in + nb);
             p += align((size_t)nb * (L.args.d + 2) * 8);
-            if (!L.args.snap) {
-                L.args.partial = p;
-                p += align((size_t)2 * L.args.n_units * L.args.N * acc_elem);
-            }
+            if (!L.args.snap) L.args.partial = static_cast<char *>(pl->dmem) + (total - partial);
             L.mats = L.args.mats;
             L.in = L.args.in;
             L.out = L.args.out;
