@@ -462,13 +462,17 @@ int grouped_plan_create(GroupedPlan *&out, const kronmult_group *groups, int n_g
         // FP64 batches of up to three rounds of entries: as many teams as share them equally.
         // (A last round of few entries waits for whole chains of barriers, and claims take about
         // 1 ns apiece: d = 2, n = 5, 200 entries 28 us with 32 teams in 4 CTAs per SM, 19 in
-        // one; d = 4, n = 4, 3000 entries 50.9 with 4 CTAs of 4 teams, 43.7 with 3.)  Entries that take less than a claim (1024
-        // operations): four per team beyond 4096 teams.
+        // one; d = 4, n = 4, 3000 entries 50.9 with 4 CTAs of 4 teams, 43.7 with 3.)  Teams that
+        // are a whole CTA: equally many on every SM, whose FP64 pipe they share (d = 6, n = 4, 1000
+        // entries 242 us with 334 CTAs, 187 with 456).  n at run time: one round only (d = 3,
+        // n = 11, 700 entries 104 us, 111 shared equally).  Entries that take less than a claim
+        // (1024 operations): four per team beyond 4096 teams.
         long long want = (long long)di.sms * per_sm * teams;
         const bool tiny = 2.0 * G.matrix_count * G.matrix_size * pow_ll(G.matrix_size, G.matrix_count) < 1024.0;
         if (dtype == KRONMULT_DTYPE_F64 && !(tunings && tunings[g].ctas_per_sm > 0)) {
             const long long rounds = (G.nb_batch + want - 1) / want;
-            if (rounds <= 3) want = (G.nb_batch + rounds - 1) / rounds;
+            if (rounds == 1 || (rounds <= 3 && !sh.snap)) want = (G.nb_batch + rounds - 1) / rounds;
+            if (rounds > 1 && teams == 1) want = (want + di.sms - 1) / di.sms * di.sms;
             if (tiny) want = std::min(want, std::max(4096LL, G.nb_batch / 4LL));
             const long long per = (want + di.sms - 1) / di.sms;  // teams per SM
             if (per < teams) {
