@@ -53,3 +53,16 @@ def test_ragged_runs_over_teams(cuda, d, n):
         want = np.asarray(O.grad_factors(b, g)).reshape(-1)
         tol = 2.0 ** -24 / math.sqrt(3) * math.sqrt((3 * d - 1) * n + n ** (d - 1) / 2 + 32 / 2 + 40 / 2)
         assert O.rel_l2(_factor_gradients(cuda, b, g).reshape(-1), want) <= tol
+
+
+@pytest.mark.parametrize("d,n,count", [(4, 6, 2411), (4, 7, 1613)])
+def test_entries_sharing_eight_warps(cuda, d, n, count):
+    """7 and 5 entries per CTA of 8 warps, several per team, runs that end at different entries."""
+    rng = np.random.Generator(np.random.PCG64(6))
+    fan = rng.integers(1, 20, size=count)
+    fan = fan[: int((np.cumsum(fan) < count).sum()) + 1]
+    fan[-1] -= fan.sum() - count
+    b = _batch(d, n, fan, 8600 + 10 * d + n)
+    g = rng.standard_normal((b.n_out, b.N))
+    want = np.asarray(O.grad_factors(b, g)).reshape(-1)
+    assert O.rel_l2(_factor_gradients(cuda, b, g).reshape(-1), want) <= 1e-5
