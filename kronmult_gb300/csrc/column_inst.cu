@@ -30,7 +30,6 @@ BlkInfo units_lookup(int n, int d1)
     if (d1 < 1 || d1 > 15) return BlkInfo{};  // the keys below hold d1 in 4 bits
     if (d1 < 1 || d1 > 15) return BlkInfo{};  // the keys below hold d1 in 4 bits
     switch (n * 16 + d1) {
-    case 2 * 16 + 7: return blk_info_of<float, BlkLarge<2, 7>, true>();
     case 2 * 16 + 8: return blk_info_of<float, BlkLarge<2, 8>, true>();
     case 2 * 16 + 9: return blk_info_of<float, BlkLarge<2, 9>, true>();
     case 2 * 16 + 10: return blk_info_of<float, BlkLarge<2, 10>, true>();
