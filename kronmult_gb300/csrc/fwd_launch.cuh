@@ -469,6 +469,9 @@ constexpr BlkSlower kBlkSlowerF32[] = {
     {7, 3, 9700, 10800},   // just beyond one wave: 0.89 of the speed there at 10000
     {7, 4, 0, 500},        // few threads per entry: 5.4 / 6.4 at 48
     {8, 4, 0, 1100},       // 14.5 / 15.1 at 1000, 31.8 / 22.1 at 2500
+    {4, 3, 7800, 9800},    // 5.8 / 6.4; 5.8 / 6.1 at 9000
+    {4, 4, 5900, 14500},   // 10.3 / 10.8; 9.3 / 10.8 at 12000, 13.5 / 11.3 at 15000
+    {4, 4, 19500, 21500},  // just beyond two waves: 13.7 / 15.4; 12.3 / 14.3 at 20000
     {4, 6, 0, 2500},       // 10.5 / 13.8 at 1000, 40.5 / 38.4 at 6000
 };
 // FP64 outputs: chunks of 6-8 entries leave a wave's last teams uneven as well
@@ -483,6 +486,7 @@ constexpr BlkSlower kBlkSlowerF64[] = {
     {7, 4, 0, 500},        // few threads per entry
     {8, 4, 0, 4000},       // 33.4 / 37.1 at 2500, 56.3 / 53.6 at 6000
     {8, 4, 7300, 9500},    // just beyond one wave: 0.84 of the speed; 0.86 at 8000
+    {4, 4, 77900, 90000},  // just beyond one wave: 0.91 of the speed; 0.85 at 80000
     {4, 5, 4000, 9500},    // two entries per output, 5000: 20.8 / 24.8
 };
 // No instantiation, for the same reason: n = 6, d = 2 (39.5 / 41.7 at 200000) and, of FP64
@@ -876,9 +880,9 @@ int plan_forward(FwdPlan<T, TO> &pl, int d, int n, const T *const *mats, int str
                 }
             }
         }
-        // FP32, n = 2, d >= 2: two modes per shared-memory pass (fwd_pair_kernel)
+        // FP32, n = 2 and 4, d >= 2: two modes per shared-memory pass (fwd_pair_kernel)
         if constexpr (sizeof(T) == 4) {
-            const bool want_pair = !single && n == 2 && d >= 2 && !(tune && tune->prefetch == 1) &&
+            const bool want_pair = !single && (n == 2 || n == 4) && d >= 2 && !(tune && tune->prefetch == 1) &&
                                    !(tune && tune->team_size > 0);
             if (want_pair) {
                 const int F2 = N / (n * n);

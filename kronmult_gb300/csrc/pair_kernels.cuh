@@ -1,5 +1,5 @@
-// FP32 forward that applies two modes per shared-memory pass (n = 2 and 8; n = 4: three,
-// d = 6 only), where it is faster than the register blocks: small batches and FP64 outputs.
+// FP32 forward that applies two modes per shared-memory pass (n = 2, 4 and 8; n = 4, d = 6: three),
+// where it is faster than the register blocks: bands of batch sizes, n = 2 into FP64 outputs.
 //
 // For FP32 the single-mode sweep is bound by shared-memory traffic (every mode
 // reads and writes the whole vector once) rather than by HBM or the FMA pipe.
@@ -12,6 +12,12 @@
 // (Y[c + r*F] twice), with the same k-ascending FMA chains.  An odd d starts with
 // one single-mode step.  Shared-memory traffic and barriers are halved.
 //
+// Bank conflicts: for n = 4 a bi-fibre is 64 bytes per lane; its four 16-byte
+// reads would hit the same banks every fourth lane.  The vector is therefore
+// stored with 16-byte chunk ch at physical chunk ch ^ ((ch >> 3) & 7): eight
+// consecutive bi-fibres then land in eight distinct bank groups, and the scalar
+// writes of 32 consecutive positions stay a permutation of one 128-byte row.
+//
 // n = 8 (team_forward_pairs8): a lane pair shares one 64-value bi-fibre X[a][b].
 // Lane h holds rows a = 4h..4h+3 and applies mode i to them (index b); the pair then
 // swaps halves with 16 shuffles so that lane h holds columns b = 4h..4h+3 of all 8
@@ -22,6 +28,27 @@
 #include "fwd_kernels.cuh"
 
 namespace kgb {
+
+template <int NN> struct PairSwizzle {
+    // physical 16-byte chunk of logical chunk ch (n = 4): the XOR of bits 3..5 keeps every
+    // aligned group of 8 chunks within itself (32 consecutive scalar positions stay one
+    // 128-byte row) and puts 8 consecutive 64-byte bi-fibres on 8 slots.  (n = 8 uses
+    // the padded layout of p8_phys instead.)
+    static __device__ __forceinline__ int chunk(int ch)
+    {
+        if constexpr (NN == 4) return ch ^ ((ch >> 3) & 7);
+        return ch;
+    }
+    // physical element index of logical element p (floats)
+    static __device__ __forceinline__ int elem(int p)
+    {
+        if constexpr (NN == 4) {
+            return (chunk(p >> 2) << 2) | (p & 3);
+        } else {
+            return p;
+        }
+    }
+};
 
 // Pointers of one entry as seen by one thread: its input vector and the factor
 // matrices of the (at most kPairFacSlots) factor elements this thread copies.
@@ -46,16 +73,16 @@ __device__ __forceinline__ void pair_load_ptrs(PairPtrs &p, const float *const *
     }
 }
 
-// stage one entry asynchronously
+// stage one entry (vector in the swizzled layout, factors plain) asynchronously
 template <int NN>
 __device__ __forceinline__ void pair_stage_async(float *dst, float *fac, const PairPtrs &p,
                                                  const float *const *mats_e, int N, int d, int stride, const Team &tm)
 {
     if (((reinterpret_cast<uintptr_t>(p.src) & 15u) == 0) && ((N & 3) == 0)) {
         for (int v = tm.rank; v < N / 4; v += tm.size)
-            cp_async<16>(dst + 4 * v, p.src + 4 * v);
+            cp_async<16>(dst + 4 * PairSwizzle<NN>::chunk(v), p.src + 4 * v);
     } else {
-        for (int v = tm.rank; v < N; v += tm.size) cp_async<4>(dst + v, p.src + v);
+        for (int v = tm.rank; v < N; v += tm.size) cp_async<4>(dst + PairSwizzle<NN>::elem(v), p.src + v);
     }
     constexpr int NN2 = NN * NN;
 #pragma unroll
@@ -82,7 +109,7 @@ __device__ __forceinline__ void team_forward_pairs(const float *const *mats, con
                                                    int d, int stride, int N, long long e_begin, long long e_end,
                                                    float *buf, float *fac, float *buf2, float *fac2, const Team &tm)
 {
-    static_assert(NN == 2, "bi-fibres of 16 bytes");
+    using SW = PairSwizzle<NN>;
     constexpr int NN2 = NN * NN;
     constexpr int Q1 = QP * NN;  // fibres per thread in a single-mode step
     const int F = N / NN, F2 = N / NN2;
@@ -115,9 +142,17 @@ __device__ __forceinline__ void team_forward_pairs(const float *const *mats, con
                 const int c = tm.rank + q * tm.size;
                 if (c < F) {
                     float xv[NN];
-                    const float2 v = *reinterpret_cast<const float2 *>(buf + 2 * c);
-                    xv[0] = v.x;
-                    xv[1] = v.y;
+                    if constexpr (NN == 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(buf + 4 * SW::chunk(c));
+                        xv[0] = v.x;
+                        xv[1] = v.y;
+                        xv[2] = v.z;
+                        xv[3] = v.w;
+                    } else {
+                        const float2 v = *reinterpret_cast<const float2 *>(buf + 2 * c);
+                        xv[0] = v.x;
+                        xv[1] = v.y;
+                    }
 #pragma unroll
                     for (int r = 0; r < NN; ++r) {
                         float s = 0.f;
@@ -128,12 +163,15 @@ __device__ __forceinline__ void team_forward_pairs(const float *const *mats, con
                 }
             }
             tm.sync();
+            // when F is a multiple of 256 the swizzle of c + r*F is the swizzle of c plus r*F
+            const bool linear1 = NN != 4 || (F & 255) == 0;
 #pragma unroll
             for (int q = 0; q < Q1; ++q) {
                 const int c = tm.rank + q * tm.size;
                 if (c < F) {
+                    const int base = SW::elem(c);
 #pragma unroll
-                    for (int r = 0; r < NN; ++r) buf[c + r * F] = y[q][r];
+                    for (int r = 0; r < NN; ++r) buf[linear1 ? base + r * F : SW::elem(c + r * F)] = y[q][r];
                 }
             }
             tm.sync();
@@ -148,46 +186,95 @@ __device__ __forceinline__ void team_forward_pairs(const float *const *mats, con
                 const int c2 = tm.rank + q * tm.size;
                 if (c2 < F2) {
                     float x[NN][NN];
-                    const float4 v = *reinterpret_cast<const float4 *>(buf + 4 * c2);
-                    x[0][0] = v.x;
-                    x[0][1] = v.y;
-                    x[1][0] = v.z;
-                    x[1][1] = v.w;
-                    // mode i on b, in place row by row
+                    if constexpr (NN == 4) {
 #pragma unroll
-                    for (int a = 0; a < NN; ++a) {
-                        float t[NN];
+                        for (int a = 0; a < 4; ++a) {
+                            const float4 v = *reinterpret_cast<const float4 *>(buf + 4 * SW::chunk(4 * c2 + a));
+                            x[a][0] = v.x;
+                            x[a][1] = v.y;
+                            x[a][2] = v.z;
+                            x[a][3] = v.w;
+                        }
+                    } else {
+                        const float4 v = *reinterpret_cast<const float4 *>(buf + 4 * c2);
+                        x[0][0] = v.x;
+                        x[0][1] = v.y;
+                        x[1][0] = v.z;
+                        x[1][1] = v.w;
+                    }
+                    if constexpr (NN == 4) {
+                        // factor columns as 16-byte broadcast loads, FMAs in packed FP32
+                        // pairs over the output index (each half the scalar k-ascending
+                        // FMA chain from 0: the same bits)
+                        const f2 zero2 = f2_pack(0.f, 0.f);
+                        // mode i on b, in place row by row; column b of M1 as rows (0,1), (2,3)
+#pragma unroll
+                        for (int a = 0; a < 4; ++a) {
+                            f2 t0 = zero2, t1 = zero2;
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) {
+                                const float4 u = *reinterpret_cast<const float4 *>(M1 + 4 * b);
+                                const f2 xb = f2_pack(x[a][b], x[a][b]);
+                                t0 = f2_fma(f2_pack(u.x, u.y), xb, t0);
+                                t1 = f2_fma(f2_pack(u.z, u.w), xb, t1);
+                            }
+                            f2_unpack(t0, x[a][0], x[a][1]);
+                            f2_unpack(t1, x[a][2], x[a][3]);
+                        }
+                        // mode i-1 on a, column by column
+#pragma unroll
+                        for (int rb = 0; rb < 4; ++rb) {
+                            f2 t0 = zero2, t1 = zero2;
+#pragma unroll
+                            for (int a = 0; a < 4; ++a) {
+                                const float4 w = *reinterpret_cast<const float4 *>(M0 + 4 * a);
+                                const f2 xa = f2_pack(x[a][rb], x[a][rb]);
+                                t0 = f2_fma(f2_pack(w.x, w.y), xa, t0);
+                                t1 = f2_fma(f2_pack(w.z, w.w), xa, t1);
+                            }
+                            f2_unpack(t0, z[q][rb], z[q][rb + 4]);
+                            f2_unpack(t1, z[q][rb + 8], z[q][rb + 12]);
+                        }
+                    } else {
+                        // mode i on b, in place row by row
+#pragma unroll
+                        for (int a = 0; a < NN; ++a) {
+                            float t[NN];
+#pragma unroll
+                            for (int rb = 0; rb < NN; ++rb) {
+                                float s = 0.f;
+#pragma unroll
+                                for (int b = 0; b < NN; ++b) s = fmaf(M1[rb + b * NN], x[a][b], s);
+                                t[rb] = s;
+                            }
+#pragma unroll
+                            for (int rb = 0; rb < NN; ++rb) x[a][rb] = t[rb];
+                        }
+                        // mode i-1 on a, column by column
 #pragma unroll
                         for (int rb = 0; rb < NN; ++rb) {
-                            float s = 0.f;
 #pragma unroll
-                            for (int b = 0; b < NN; ++b) s = fmaf(M1[rb + b * NN], x[a][b], s);
-                            t[rb] = s;
-                        }
+                            for (int ra = 0; ra < NN; ++ra) {
+                                float s = 0.f;
 #pragma unroll
-                        for (int rb = 0; rb < NN; ++rb) x[a][rb] = t[rb];
-                    }
-                    // mode i-1 on a, column by column
-#pragma unroll
-                    for (int rb = 0; rb < NN; ++rb) {
-#pragma unroll
-                        for (int ra = 0; ra < NN; ++ra) {
-                            float s = 0.f;
-#pragma unroll
-                            for (int a = 0; a < NN; ++a) s = fmaf(M0[ra + a * NN], x[a][rb], s);
-                            z[q][rb + NN * ra] = s;
+                                for (int a = 0; a < NN; ++a) s = fmaf(M0[ra + a * NN], x[a][rb], s);
+                                z[q][rb + NN * ra] = s;
+                            }
                         }
                     }
                 }
             }
             tm.sync();  // every read of buf (and fac) for this pass is done
             if (i > 1) {
+                // when F2 is a multiple of 256 the swizzle of c2 + j*F2 is the swizzle of c2 plus j*F2
+                const bool linear2 = NN != 4 || (F2 & 255) == 0;
 #pragma unroll
                 for (int q = 0; q < QP; ++q) {
                     const int c2 = tm.rank + q * tm.size;
                     if (c2 < F2) {
+                        const int base = SW::elem(c2);
 #pragma unroll
-                        for (int j = 0; j < NN2; ++j) buf[c2 + F2 * j] = z[q][j];
+                        for (int j = 0; j < NN2; ++j) buf[linear2 ? base + F2 * j : SW::elem(c2 + F2 * j)] = z[q][j];
                     }
                 }
                 tm.sync();
@@ -823,6 +910,8 @@ template <typename TO> FwdSmemFn<float, TO> fwd_pair_lookup(int nn, int qp);
         switch (nn * 16 + qp) {                                                                        \
         case 2 * 16 + 1: return fwd_pair_kernel<TO, 2, 1>;                                             \
         case 2 * 16 + 2: return fwd_pair_kernel<TO, 2, 2>;                                             \
+        case 4 * 16 + 1: return fwd_pair_kernel<TO, 4, 1>;                                             \
+        case 4 * 16 + 2: return fwd_pair_kernel<TO, 4, 2>;                                             \
         case 8 * 16 + 1: return fwd_pair8_kernel<TO>;                                                  \
         case 4 * 16 + 3: return fwd_tri4_kernel<TO>; /* d = 6: three modes per pass */                 \
         default: return nullptr;                                                                       \

@@ -136,3 +136,16 @@ def test_two_streams(cuda):
         adjoint(blk, gout, gin, gfa, stream=streams[0])
         for a, b in zip(results(), want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("d,nb", [(3, 9001), (4, 12007)])
+def test_pairs_bitwise(cuda, d, nb):
+    """n = 4 in a band of batch sizes that the register blocks leave to the bi-fibre kernel."""
+    b = _batch(cuda, d, 4, nb, torch.float32)
+    assert "fwd_pair_kernel" in planned_kernel(d, 4, F32, nb)
+    b.forward()
+    got = b.outputs.clone()
+    b.outputs.zero_()
+    b.forward(tuning={"team_size": 256})
+    torch.cuda.synchronize()
+    assert torch.equal(got, b.outputs)
