@@ -11,7 +11,7 @@
 //
 // What bounds it: the FP64 pipe for large batches (1.0-1.19 of 1.25 TFLOP/s), the 3 d phases'
 // barriers and dependent additions for small ones.  Against the element kernels with a
-// power-of-two team per entry: d = 3, n = 6 820 -> 720 us at 40000 entries, 20.4 -> 7.3 at 16;
+// power-of-two team per entry: d = 3, n = 6 820 -> 735 us at 40000 entries, 20.4 -> 7.3 at 16;
 // d = 4, n = 8 1058 -> 716 at 1000; d = 2, n = 4 43 -> 28 at 40000; d = 4, n = 4 20.9 -> 8.1 at
 // 16.
 #pragma once

@@ -29,11 +29,11 @@
 // threads own consecutive positions.
 //
 // Measured against the kernels that apply one mode (n = 2, 4, 8: two) per shared-memory pass,
-// FP32: d = 4, n = 5, 35007 entries 89.6 -> 45.8 us (DRAM sectors 67 % of peak at a stride of
-// 67); d = 6, n = 4, 36864 entries 207 -> 191 us; d = 2, n = 3, 200000 entries 34.9 -> 19.1; d = 3,
-// n = 6, 200000 entries 160 -> 100; FP64 outputs, d = 4, n = 8, 32768 entries 268 -> 225 us.  With
-// 64 values per thread (168 registers, 12 warps per SM) the FMA pipe is 48-56 % busy and DRAM
-// 46-54 %: register-port conflicts stall dispatch for about a quarter of the cycles.
+// FP32: d = 4, n = 5, 35007 entries 89.6 -> 46.4 us (DRAM sectors 67 % of peak at a stride of
+// 67); d = 6, n = 4, 36864 entries 207 -> 200 us; d = 2, n = 3, 200000 entries 34.9 -> 19.8; d = 3,
+// n = 6, 200000 entries 160 -> 100; FP64 outputs, d = 4, n = 8, 32768 entries 268 -> 219 us.  With
+// 64 values per thread (168 registers, 12 warps per SM) the FMA pipe is 45-56 % busy and DRAM
+// 45-54 %: register-port conflicts stall dispatch for about a quarter of the cycles.
 #pragma once
 #include <type_traits>
 #include "fwd_kernels.cuh"

@@ -439,13 +439,11 @@ template <typename TO> bool block_chunks(FwdArgs<float, TO> &a, const DeviceInfo
 
 // Where the other FP32 kernels measured faster than the register blocks: [from, to) entries.
 // Most lie where a batch is a few waves of small teams and their uneven last one costs what
-// the blocks save.  Figures: us there / in register blocks at the entries named, one output
-// per entry and (after the semicolon) one per 8 entries.  Left as they are: large batches of
-// one output per entry, whose stores the persistent teams spread over all of memory (d = 6,
-// n = 4, 30000 entries 220 / 244; FP64 outputs, d = 4, n = 8 398 / 440), where two or more
-// entries per output gain (183 / 167 and 294 / 274 at two, 171 / 155 and 247 / 221 at eight):
-// the host cannot tell them apart, and taking the entries in batch order where the outputs
-// lie apart gained 4 % there and cost 1-8 % everywhere else (registers).
+// the blocks save, or just beyond a whole number of waves.  Figures: us there / in register
+// blocks at the entries named, one output per entry and (after the semicolon) one per 8
+// entries.  Left as they are: batches where one entry per output loses what more gain (FP64
+// outputs, d = 3, n = 7, 60000 entries 129 / 172 at one, 1.23 times as fast at eight): the host
+// cannot tell them apart.
 struct BlkSlower {
     int n, d;
     long long from, to;
